@@ -672,6 +672,13 @@ int nd_selftest_exact_add(const double* a, const double* b, double* out, int64_t
     return err == cudaSuccess ? ND_OK : cuda_fail(err, "nd_selftest_exact_add");
 }
 
+int nd_selftest_trig(const double* x, double* s, double* c, int64_t n, void* stream) {
+    clear_error();
+    if (n < 0 || (n > 0 && (!x || !s || !c))) return fail(ND_ERR_ARG, "nd_selftest_trig: bad arguments");
+    cudaError_t err = launch_trig_selftest(x, s, c, n, (cudaStream_t)stream);
+    return err == cudaSuccess ? ND_OK : cuda_fail(err, "nd_selftest_trig");
+}
+
 int nd_selftest_exact_scan(const double* terms, const int64_t* seg, const double* s0, double* out, int64_t nseg,
                            void* stream) {
     clear_error();

@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "nd_gb300.h"
+#include "nd_trig.cuh"
 
 namespace nd {
 
@@ -19,9 +20,10 @@ struct Arith<double> {
     static __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
     static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
     static __device__ __forceinline__ double div(double a, double b) { return __ddiv_rn(a, b); }
-    // FP64 keeps the raw phase difference, like the reference's sin(θs - θd).
-    static __device__ __forceinline__ double sin_phase(double x) { return sin(x); }
-    static __device__ __forceinline__ double cos_phase(double x) { return cos(x); }
+    // FP64 keeps the raw phase difference, like the reference's sin(θs - θd); both functions
+    // run on the integer pipes (nd_trig.cuh).
+    static __device__ __forceinline__ double sin_phase(double x) { return trig::sin(x); }
+    static __device__ __forceinline__ double cos_phase(double x) { return trig::cos(x); }
 };
 
 // 2π split for a two-step Cody–Waite reduction of a phase difference to [-π, π].

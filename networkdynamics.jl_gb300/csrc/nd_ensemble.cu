@@ -473,7 +473,7 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
                     const int32_t eb = a.eid[k];
                     const double Kk = EK == ND_E_DIFFUSION_UNIT ? 1.0 : pe[eb & 0x7fffffff];
                     const double dth = th[2 * (int64_t)a.nbr[k]] - uv;
-                    W[k] = EK == ND_E_KURAMOTO ? Kk * cos(dth) : Kk;
+                    W[k] = EK == ND_E_KURAMOTO ? Kk * A::cos_phase(dth) : Kk;
                 }
                 X[s.vbase + v] = 0.0;
                 R[s.vbase + v] = G[s.vbase + v];

@@ -356,6 +356,15 @@ __global__ void exact_add_selftest_kernel(const double* a, const double* b, doub
     if (i < n) out[i] = exact::add_rn(a[i], b[i]);
 }
 
+// Self-test of the fixed-point sine and cosine.
+__global__ void trig_selftest_kernel(const double* x, double* s, double* c, int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        s[i] = trig::sin(x[i]);
+        c[i] = trig::cos(x[i]);
+    }
+}
+
 // Self-test of the exact scans: one block per segment; odd segments use the 32-term warp
 // scan on registers, even segments shared-memory tiles with the 32-term scan (w % 4 == 2)
 // or the sliding 256-term scan of the heavy rows' path (w % 4 == 0).
@@ -395,6 +404,12 @@ cudaError_t launch_rhs(int dtype, const RhsArgs& a, cudaStream_t s) {
 cudaError_t launch_exact_selftest(const double* a, const double* b, double* out, int64_t n, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     exact_add_selftest_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, b, out, n);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_trig_selftest(const double* x, double* s, double* c, int64_t n, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    trig_selftest_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x, s, c, n);
     return cudaGetLastError();
 }
 
