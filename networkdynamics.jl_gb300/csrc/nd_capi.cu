@@ -165,11 +165,22 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
     // light rows in runs of consecutive vertices, are cut into windows of at most kWindow
     // rows and kWindowIncidences incidences and sorted by degree (descending, stable)
     // inside each window.
+    const bool canonical = edge_elem > 0 && ne > 0 && is_canonical(ne, src, dst);
+    int64_t heavy_min = kMediumMaxDeg + 1;
+    if (edge_elem == 8 && canonical) {
+        // not where rows that long are the bulk of the network (a dense graph: its rows have a
+        // kernel of their own)
+        const int64_t h = heavy_min_deg(2 * ne);
+        int64_t inc = 0;
+        for (int64_t v = 0; v < nv; ++v)
+            if (deg[v] >= (uint32_t)h) inc += deg[v];
+        if (8 * inc <= 2 * ne) heavy_min = h;
+    }
     std::vector<int32_t> light, medium, heavy;
     light.reserve(nv);
     for (int64_t v = 0; v < nv; ++v) {
         if (deg[v] <= (uint32_t)kLightMaxDeg) light.push_back((int32_t)v);
-        else if (deg[v] <= (uint32_t)kMediumMaxDeg) medium.push_back((int32_t)v);
+        else if (deg[v] < (uint32_t)heavy_min) medium.push_back((int32_t)v);
         else heavy.push_back((int32_t)v);
     }
     auto by_degree = [&](int32_t a, int32_t b) { return deg[a] > deg[b]; };
@@ -243,7 +254,7 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
         free_topology(&t);
         return cuda_fail(err, "upload of the network topology");
     }
-    if (edge_elem > 0 && ne > 0 && is_canonical(ne, src, dst)) {
+    if (canonical) {
         EdgeLayoutHost h;
         build_edge_layout(nv, ne, src, dst, h);
         // the row records and the padded loc array, in slot order of the rows

@@ -76,6 +76,16 @@ inline int edge_outdim(int ek) { return ek == ND_E_PILINE ? 2 : 1; }
 // a per-thread chain that long would wait on the shared FP64 pipe at every step.
 constexpr int kLightMaxDeg = 32;
 constexpr int kMediumMaxDeg = 2048;
+// Shortest heavy row of an FP64 handle's two-phase layout with ninc incidences.  A thread sums
+// a row at about 80 ns a term (one memory round trip per batch of 12), so on a small network
+// the row phase lasts as long as its longest row, while all rows together take about 4 ns per
+// 1000 incidences (327 µs for the 8e7 of BA(1e7, 4)).  Rows above the length that costs the
+// thread half of that go to the heavy kernel, which starts beside the edge phase; below 128
+// terms (10 µs) the launch on the side stream is not worth it.
+constexpr int64_t heavy_min_deg(int64_t ninc) {
+    const int64_t d = ninc / 40000;
+    return 1 + (d < 128 ? 128 : (d > kMediumMaxDeg ? kMediumMaxDeg : d));
+}
 constexpr int kWindow = 256;
 constexpr int kWarpRowMinF32 = 128;  // FP32 rows at least this long take a warp in the row phase
 constexpr int kLightRun = 128;

@@ -201,14 +201,11 @@ __global__ void __launch_bounds__(kBlock, 8) rhs_kernel(RhsArgs a) {
 // serial, and on a crowded SM each of its steps waits for other blocks' instructions.
 constexpr int kHeavySoloSmem = 160 * 1024;
 
-// FP64 sequential sum of a heavy row in the solo kernel, in tiles of TILE terms: warp 0
-// adds tile k of the row's terms (exact scan, or the hardware DADD chain in the native
-// mode) while warps 1..7 evaluate tile k + 1 into the other half of a double buffer, so the
-// serial chain never waits for its terms after the first tile.
-constexpr int kSoloTile = 8192;
-
-template <int VK, int EK, int MODE, int TILE>
-__device__ __forceinline__ void solo_row_fp64(const RhsArgs& a, int slot, double* buf) {
+// FP64 sequential sum of a heavy row by one block: tiles of kBlockTile terms, each added by the
+// block-wide exact scan (or the hardware DADD chain in the native mode).  A thread's incidence
+// data of the next tile are in flight while the current tile is added.
+template <int VK, int EK, int MODE>
+__device__ __forceinline__ void solo_row_fp64(const RhsArgs& a, int slot, double* tile, BlockScanShared& sh) {
     constexpr int DV = VertexDims<VK>::dim;
     const double* __restrict__ u = static_cast<const double*>(a.u);
     const double* __restrict__ p = static_cast<const double*>(a.p);
@@ -218,83 +215,73 @@ __device__ __forceinline__ void solo_row_fp64(const RhsArgs& a, int slot, double
     const int64_t v = __ldg(a.slot_vertex + slot);
     const uint32_t beg = __ldg(a.slot_ptr + slot), end = __ldg(a.slot_ptr + slot + 1);
     const double uv = __ldg(u + v * DV);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int ntiles = (int)((end - beg + TILE - 1) / TILE);
-    auto load = [&](int k, int first, int stride) {
-        const uint32_t base = beg + (uint32_t)k * TILE;
-        const int n = (int)min((uint32_t)TILE, end - base);
-        double* dst = buf + (k & 1) * TILE;
-#pragma unroll 4
-        for (int i = first; i < n; i += stride) {
-            const int2 inc = ld_hint(incid + base + i, stream);
-            const double un = ld_hint(u + (int64_t)inc.x * DV, keep);
-            const double w = edge_param<double, EK>(pe, inc.y & 0x7fffffff, stream);
-            dst[i] = incidence_term_w<double, EK>(uv, un, w, inc.y < 0);
+    const int tid = threadIdx.x;
+    double un[kBlockPer], w[kBlockPer];
+    unsigned src_side = 0;
+    auto load = [&](uint32_t base) {  // positions tid, tid + kBlock, ...: coalesced
+        src_side = 0;
+#pragma unroll
+        for (int k = 0; k < kBlockPer; ++k) {
+            const uint32_t i = base + (uint32_t)(tid + k * kBlock);
+            un[k] = w[k] = 0.0;
+            if (i < end) {
+                const int2 inc = ld_hint(incid + i, stream);
+                un[k] = ld_hint(u + (int64_t)inc.x * DV, keep);
+                w[k] = edge_param<double, EK>(pe, inc.y & 0x7fffffff, stream);
+                src_side |= (unsigned)(inc.y < 0) << k;
+            }
         }
     };
-    if (ntiles > 0) load(0, tid, kBlock);
-    __syncthreads();
+    load(beg);
     double S = 0.0;
-    for (int k = 0; k < ntiles; ++k) {
-        if (warp == 0) {
-            const double* cur = buf + (k & 1) * TILE;
-            const int n = (int)min((uint32_t)TILE, end - (beg + (uint32_t)k * TILE));
-            if constexpr (MODE == kModeNative) {
-                if (lane == 0)
-                    for (int i = 0; i < n; ++i) S = __dadd_rn(S, cur[i]);
-            } else {
-                S = exact_scan_wide(S, cur, n, lane);
-            }
-        } else if (k + 1 < ntiles) {
-            load(k + 1, tid - 32, kBlock - 32);
+    for (uint32_t base = beg; base < end; base += kBlockTile) {
+        const int n = (int)min((uint32_t)kBlockTile, end - base);
+#pragma unroll
+        for (int k = 0; k < kBlockPer; ++k)
+            if (tid + k * kBlock < n)
+                tile[tile_at(tid + k * kBlock)] = incidence_term_w<double, EK>(uv, un[k], w[k], (src_side >> k) & 1u);
+        __syncthreads();
+        load(base + kBlockTile);
+        if constexpr (MODE == kModeNative) {
+            if (tid < 32)
+                for (int i = 0; i < n; ++i) S = __dadd_rn(S, tile[tile_at(i)]);
+        } else {
+            S = exact_scan_block(S, tile, n, sh);
         }
         __syncthreads();
     }
     if (tid == 0) vertex_f<double, VK>(static_cast<double*>(a.du), u, p, v, S);
 }
 
-template <typename T, int VK, int EK, int MODE, int TILE>
+template <typename T, int VK, int EK, int MODE>
 __global__ void __launch_bounds__(kBlock, 1) heavy_solo_kernel(RhsArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_dyn[];
     if constexpr (sizeof(T) == 8 && MODE != kModeTree) {
-        static_assert(2 * TILE * sizeof(double) <= kHeavySoloSmem, "solo double buffer");
-        solo_row_fp64<VK, EK, MODE, TILE>(a, blockIdx.x, reinterpret_cast<double*>(smem_dyn));
+        __shared__ double tile[kBlockTilePadded];
+        __shared__ BlockScanShared sh;
+        solo_row_fp64<VK, EK, MODE>(a, blockIdx.x, tile, sh);
     } else {
+        extern __shared__ __align__(16) unsigned char smem_dyn[];
         block_row<T, VK, EK, MODE>(a, blockIdx.x, smem_dyn);
     }
 }
 
-template <typename T, int VK, int EK, int MODE, int TILE>
-cudaError_t launch_heavy_solo_t(const RhsArgs& a, cudaStream_t s, int smem) {
-    static int attr_set = 0;  // per instantiation; the attribute is per function
-    if (attr_set < smem) {
-        cudaError_t err = cudaFuncSetAttribute(heavy_solo_kernel<T, VK, EK, MODE, TILE>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (err != cudaSuccess) return err;
-        attr_set = smem;
-    }
-    heavy_solo_kernel<T, VK, EK, MODE, TILE><<<a.n_heavy, kBlock, smem, s>>>(a);
-    return cudaGetLastError();
-}
-
-// The FP64 sequential sums (exact scan and hardware chains) use tiles of kSoloTileShared
-// terms: 32 KB of shared memory, so that a heavy-row block also fits on an SM that already
-// holds seven edge-phase blocks.  With the whole-SM request a heavy block could start only
-// on an SM holding at most four, and when the edge phase had filled the GPU first the heavy
-// rows waited for its end and outlasted the row phase: stretches of calls at 776-793 µs
-// instead of 755 µs on BA(1e7, 4).  With the small tiles and the handle's high-priority
-// side stream (FP64 handles) the step took 747-753 µs in every stretch.  The FP32 and tree
-// heavy rows keep the whole-SM request: with small tiles they took 515 µs against 476 µs.
-constexpr int kSoloTileShared = 2048;
-
+// The FP64 sequential rows ask for 18 KB of shared memory, so that a block also fits on an SM
+// that holds several edge-phase blocks; they run on the handle's high-priority side stream.
+// The FP32 and tree rows ask for most of an SM (kHeavySoloSmem).
 template <typename T, int VK, int EK, int MODE>
 cudaError_t launch_heavy_solo(const RhsArgs& a, cudaStream_t s) {
-    if constexpr (sizeof(T) == 8 && MODE != kModeTree) {
-        constexpr int smem = (int)(2 * kSoloTileShared * sizeof(double));
-        return launch_heavy_solo_t<T, VK, EK, MODE, kSoloTileShared>(a, s, smem);
-    } else {
-        return launch_heavy_solo_t<T, VK, EK, MODE, kSoloTile>(a, s, kHeavySoloSmem);
+    constexpr int smem = sizeof(T) == 8 && MODE != kModeTree ? 0 : kHeavySoloSmem;
+    if constexpr (smem > 0) {
+        static int attr_set = 0;  // per instantiation; the attribute is per function
+        if (attr_set < smem) {
+            cudaError_t err = cudaFuncSetAttribute(heavy_solo_kernel<T, VK, EK, MODE>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (err != cudaSuccess) return err;
+            attr_set = smem;
+        }
     }
+    heavy_solo_kernel<T, VK, EK, MODE><<<a.n_heavy, kBlock, smem, s>>>(a);
+    return cudaGetLastError();
 }
 
 template <typename T, int VK, int EK>
@@ -366,11 +353,12 @@ __global__ void trig_selftest_kernel(const double* x, double* s, double* c, int6
 }
 
 // Self-test of the exact scans: one block per segment; odd segments use the 32-term warp
-// scan on registers, even segments shared-memory tiles with the 32-term scan (w % 4 == 2)
-// or the sliding 256-term scan of the heavy rows' path (w % 4 == 0).
+// scan on registers, even segments shared-memory tiles with the 32-term scan (w % 4 == 2),
+// the sliding 256-term scan (w % 8 == 0) or the block-wide scan of the heavy rows (w % 8 == 4).
 __global__ void exact_scan_selftest_kernel(const double* terms, const int64_t* seg, const double* s0, double* out,
                                            int64_t nseg) {
-    __shared__ double tile[kTile];
+    __shared__ double tile[kBlockTilePadded];
+    __shared__ BlockScanShared sh;
     const int64_t w = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double S = s0[w];
@@ -382,6 +370,14 @@ __global__ void exact_scan_selftest_kernel(const double* terms, const int64_t* s
                 const int n = (int)min((int64_t)32, seg[w + 1] - c);
                 S = exact_scan_add(S, t, n, lane);
             }
+        }
+    } else if ((w & 7) == 4) {
+        for (int64_t base = seg[w]; base < seg[w + 1]; base += kBlockTile) {
+            const int n = (int)min((int64_t)kBlockTile, seg[w + 1] - base);
+            for (int i = threadIdx.x; i < n; i += blockDim.x) tile[tile_at(i)] = terms[base + i];
+            __syncthreads();
+            S = exact_scan_block(S, tile, n, sh);
+            __syncthreads();
         }
     } else {
         for (int64_t base = seg[w]; base < seg[w + 1]; base += kTile) {

@@ -340,5 +340,258 @@ static __device__ __forceinline__ double exact_scan_wide(double S, const double*
 }
 
 
+// ---- the same sum by a whole block ------------------------------------------------------------
+// A long row is one chain of dependent roundings: 63 clocks a term with hardware adds on an
+// idle SM (several times that beside other FP64 work, which shares the SM's one FP64 unit), and
+// a restart of the scan above at every binade change, which a sum of mixed signs has every few
+// terms.  Here a block takes kBlockTile terms a step on the integer pipes, across binade changes:
+//   1. approximate prefix sums (fixed point, one scan) predict the binade of every running sum;
+//   2. with S_i in units of 2^-9 ulps of the frame's top binade, and g_i the ulp of S_i's
+//      predicted binade in that unit,
+//          S_i = g_i · RNE((S_{i-1} + t_i) / g_i).
+//      Where g_i <= g_{i-1} and t_i is not halfway between multiples of g_i, that is S_{i-1} plus
+//      t_i rounded to g_i, whatever S_{i-1} is: a second scan adds these.  The others, "events"
+//      (ties, and steps into a higher binade, which round S_{i-1}'s own last bits), are few;
+//   3. one warp goes through the events in order (an integer add, a rounding and a subtraction
+//      each, about 50 clocks) and hands every position the correction of the last event before it;
+//   4. every position checks that its sum lies strictly inside its predicted binade: up to the
+//      first that does not, all are the sequential sum's bits, by induction.
+// The frame spans 8 binades (the starting sum's, four above, three below).  A step ends at the
+// first position outside it, after which a few terms take hardware adds.
+// Measured as the heavy kernel beside the edge phase: BA(2e6, 4) diffusion 217 µs -> 80 µs (the
+// warp scan on its 9 rows above 2048 terms against this one on all 264 from 400 up; the largest
+// has 6327), BA(1e5, 2) swing 47 µs for its 36 rows above 128 (the largest has 935; a thread
+// takes 56 to 75 µs for it, and the 256-term scan restarted at binade changes took 92 µs).
+constexpr int kBlockPer = 4;
+constexpr int kBlockTile = kBlock * kBlockPer;
+// Position i of a tile in shared memory: one pad entry per thread's terms keeps the threads'
+// reads of their own terms free of bank conflicts.
+__device__ __forceinline__ int tile_at(int i) { return i + i / kBlockPer; }
+constexpr int kBlockTilePadded = kBlockTile + kBlockTile / kBlockPer;
+constexpr int kFrameUp = 4, kFrameTop = 9, kFrameLow = 2;  // log2 of g: kFrameTop in the top binade
+
+struct BlockScanShared {
+    int64_t approx[kWarpsPerBlock], total[kWarpsPerBlock];
+    int count[kWarpsPerBlock], emax[kWarpsPerBlock];
+    unsigned outside[kWarpsPerBlock], first_bad[kWarpsPerBlock];
+    int n_events;
+    double sum;
+    // events: the prefix before it (then the correction behind it), its term, log2 g
+    int64_t ev_prefix[kBlockTile], ev_term[kBlockTile];
+    int8_t ev_shift[kBlockTile];
+};
+
+__device__ __forceinline__ int64_t signed_of(uint64_t mag, uint64_t bits) {
+    return (bits & exact::kSign) ? -(int64_t)mag : (int64_t)mag;
+}
+
+// S + the n terms of `tile` (tile_at layout), in order; S is the same in every thread, and so
+// is the result.  All kBlock threads call it; `tile` is visible to all of them before.
+static __device__ __forceinline__ double exact_scan_block(double S, const double* __restrict__ tile, int n,
+                                                          BlockScanShared& sh) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int base = tid * kBlockPer;
+    // this thread's terms: significands, exponent fields (subnormals: 1) and signs
+    uint64_t mag[kBlockPer], bits[kBlockPer];
+    int et[kBlockPer];
+    int emax = 0;
+#pragma unroll
+    for (int i = 0; i < kBlockPer; ++i) {
+        bits[i] = base + i < n ? exact::to_bits(tile[tile_at(base + i)]) : 0;
+        const int e = (int)((bits[i] >> 52) & 0x7ff);
+        mag[i] = (bits[i] & exact::kFrac) | (e ? exact::kHidden : 0);
+        et[i] = e ? e : 1;
+        emax = max(emax, e);
+    }
+    emax = (int)__reduce_max_sync(kFull, (unsigned)emax);
+    if (lane == 0) sh.emax[warp] = emax;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kWarpsPerBlock; ++w) emax = max(emax, sh.emax[w]);
+    int pos = 0, run_len = 8;
+    // > 0: the next run is this many hardware adds.  All of a tile with infinities or NaN; the
+    // first terms of a row, whose sum starts at zero.
+    int fallback = emax == 0x7ff ? n : ((exact::to_bits(S) << 1) == 0 ? run_len : 0);
+    while (pos < n) {
+        const uint64_t sb = exact::to_bits(S);
+        const int eS = (int)((sb >> 52) & 0x7ff);
+        if (fallback == 0 && (eS < 16 || eS > 0x7ff - 32)) fallback = 1;  // zero, subnormal, near overflow, not finite
+        if (fallback > 0) {  // one warp, so that the SM's FP64 unit serves this chain alone
+            const int stop = min(n, pos + fallback);
+            if (warp == 0) {
+                for (int i = pos; i < stop; ++i) S = __dadd_rn(S, tile[tile_at(i)]);
+                if (lane == 0) sh.sum = S;
+            }
+            __syncthreads();
+            S = sh.sum;
+            __syncthreads();
+            pos = stop;
+            fallback = 0;
+            continue;
+        }
+        // 1. approximate prefix sums in units of 2^(EA - 1085): at most 1025 numbers below
+        //    2^(EA - 1034), so no sum overflows
+        const int EA = max(eS, emax) + 12;
+        const uint64_t magS = (sb & exact::kFrac) | exact::kHidden;
+        const int64_t aS = signed_of(magS >> min(63, EA - eS - 10), sb);
+        int64_t apx[kBlockPer];
+        int64_t run = 0;
+#pragma unroll
+        for (int i = 0; i < kBlockPer; ++i) {
+            if (base + i >= pos) run += signed_of(mag[i] >> min(63, EA - et[i] - 10), bits[i]);
+            apx[i] = run;
+        }
+        int64_t x = run;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int64_t y = __shfl_up_sync(kFull, x, off);
+            if (lane >= off) x += y;
+        }
+        if (lane == 31) sh.approx[warp] = x;
+        __syncthreads();
+        int64_t before = aS + (x - run);
+        for (int w = 0; w < warp; ++w) before += sh.approx[w];
+        // 2. predicted log2 g, rounded terms and events
+        auto log_g = [&](int64_t A) {  // of the binade of an approximate sum; 0: too small to tell
+            const uint64_t m = (uint64_t)(A < 0 ? -A : A);
+            if (m < (1ull << 22)) return 0;
+            const int e = EA - 62 + 63 - exact::clz64(m);
+            return max(0, min(kFrameTop + 1, e - eS + (kFrameTop - kFrameUp)));
+        };
+        int64_t term[kBlockPer], pre[kBlockPer];
+        int lg[kBlockPer];
+        unsigned events = 0, outside = 0xffffffffu;
+        int prev = max(kFrameLow, min(kFrameTop, log_g(before)));
+        run = 0;
+#pragma unroll
+        for (int i = 0; i < kBlockPer; ++i) {
+            const int q = base + i;
+            lg[i] = log_g(before + apx[i]);
+            const int L = et[i] - eS + (kFrameTop - kFrameUp);  // t in frame units: significand · 2^L
+            const bool active = q >= pos && q < n;
+            if (active && (lg[i] < kFrameLow || lg[i] > kFrameTop || (L > 10 && mag[i] != 0))) outside = min(outside, (unsigned)q);
+            uint64_t m;
+            if (L >= 0) {
+                m = mag[i] << min(L, 10);
+            } else {  // the bits below the unit only count as "not zero" (the last bit set)
+                const int r = min(-L, 63);
+                m = mag[i] >> r;
+                m |= (uint64_t)((m << r) != mag[i]);
+            }
+            term[i] = active ? signed_of(m, bits[i]) : 0;
+            const int s = max(kFrameLow, min(kFrameTop, lg[i]));
+            const uint32_t g = 1u << s, low = (uint32_t)term[i] & (g - 1);
+            const bool event = active && (lg[i] > prev || low == g / 2);
+            events |= (unsigned)event << i;
+            if (!event) run += (term[i] + (int64_t)(g / 2)) & ~(int64_t)(g - 1);
+            pre[i] = run;
+            lg[i] = s;
+            prev = s;
+        }
+        x = run;
+        int cnt = __popc(events);
+        const int mine = cnt;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int64_t y = __shfl_up_sync(kFull, x, off);
+            const int c = __shfl_up_sync(kFull, cnt, off);
+            if (lane >= off) {
+                x += y;
+                cnt += c;
+            }
+        }
+        outside = __reduce_min_sync(kFull, outside);
+        if (lane == 31) {
+            sh.total[warp] = x;
+            sh.count[warp] = cnt;
+            sh.outside[warp] = outside;
+        }
+        __syncthreads();
+        before = x - run;
+        cnt -= mine;
+        int P = n;
+#pragma unroll
+        for (int w = 0; w < kWarpsPerBlock; ++w) {
+            if (w < warp) {
+                before += sh.total[w];
+                cnt += sh.count[w];
+            }
+            P = (int)min((unsigned)P, sh.outside[w]);
+        }
+        // the events before the first position outside the frame, in order
+        int idx = cnt;
+#pragma unroll
+        for (int i = 0; i < kBlockPer; ++i) {
+            if (((events >> i) & 1u) && base + i < P) {
+                sh.ev_prefix[idx] = before + pre[i];
+                sh.ev_term[idx] = term[i];
+                sh.ev_shift[idx] = (int8_t)lg[i];
+                ++idx;
+            }
+        }
+        if (P > base && P <= base + kBlockPer) sh.n_events = idx;
+        if (P == 0 && tid == 0) sh.n_events = 0;
+        __syncthreads();
+        // 3. the events, in order
+        const int64_t m0 = signed_of(magS << (kFrameTop - kFrameUp), sb);
+        if (warp == 0) {
+            const int ne = sh.n_events;
+            int64_t c = m0;
+            int64_t b = sh.ev_prefix[0], t = sh.ev_term[0];
+            int s = sh.ev_shift[0];
+            for (int k = 0; k < ne; ++k) {
+                const int kn = min(k + 1, kBlockTile - 1);
+                const int64_t bn = sh.ev_prefix[kn], tn = sh.ev_term[kn];
+                const int sn = sh.ev_shift[kn];
+                const int64_t v = c + (b + t);
+                const uint32_t g = 1u << s, lsb = ((uint32_t)v >> s) & 1u;
+                c = ((v + (int64_t)(g / 2 - 1 + lsb)) & ~(int64_t)(g - 1)) - b;
+                __syncwarp();
+                if (lane == 0) sh.ev_prefix[k] = c;
+                b = bn;
+                t = tn;
+                s = sn;
+            }
+        }
+        __syncthreads();
+        // 4. the sums, and the first position whose sum is not strictly inside its binade
+        int64_t val[kBlockPer];
+        unsigned firstbad = 0xffffffffu;
+#pragma unroll
+        for (int i = 0; i < kBlockPer; ++i) {
+            cnt += (int)((events >> i) & 1u);
+            const bool in = base + i >= pos && base + i < P;
+            val[i] = before + pre[i] + (cnt > 0 && in ? sh.ev_prefix[cnt - 1] : m0);
+            const uint64_t am = (uint64_t)(val[i] < 0 ? -val[i] : val[i]) >> lg[i];
+            if (in && (am < (1ull << 52) + 1 || am > (1ull << 53) - 2)) firstbad = min(firstbad, (unsigned)(base + i));
+        }
+        firstbad = __reduce_min_sync(kFull, firstbad);
+        if (lane == 0) sh.first_bad[warp] = firstbad;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kWarpsPerBlock; ++w) P = (int)min((unsigned)P, sh.first_bad[w]);
+        // positions [pos, P) are exact: the owner of P - 1 publishes the sum behind it
+        if (P > pos) {
+#pragma unroll
+            for (int i = 0; i < kBlockPer; ++i)
+                if (base + i == P - 1) {
+                    const uint64_t am = (uint64_t)(val[i] < 0 ? -val[i] : val[i]) >> lg[i];
+                    sh.sum = exact::from_bits((val[i] < 0 ? exact::kSign : 0) |
+                                              ((uint64_t)(eS + lg[i] - (kFrameTop - kFrameUp)) << 52) |
+                                              (am & exact::kFrac));
+                }
+            __syncthreads();
+            S = sh.sum;
+        }
+        // behind a position outside the frame a run of hardware adds, longer while steps stay short
+        run_len = P - pos >= 64 ? 4 : min(64, 2 * run_len);
+        pos = P;
+        if (pos < n) fallback = run_len;
+        __syncthreads();  // sh is written again
+    }
+    return S;
+}
+
+
 }  // namespace dev
 }  // namespace nd

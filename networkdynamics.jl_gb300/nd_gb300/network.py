@@ -42,8 +42,8 @@ class GB300Execution(ExecutionStyle):
     - ``kernel_timing``: bracket every kernel with CUDA events for ``Network.kernel_times``.
 
     The precision is the dtype given to ``adapt``.  The degree buckets (light rows up to 32,
-    heavy rows above 2048) and the FP32 Kahan threshold (rows longer than 32) are
-    compile-time constants of the kernels."""
+    heavy rows above 2048, in FP64 already above 128 to 2048 terms by the network's size) and
+    the FP32 Kahan threshold (rows longer than 32) are constants of the library."""
 
     buffered = False
     SUM_ORDERS = ("sequential", "sequential_hw", "tree")
