@@ -22,6 +22,9 @@ int nd_selftest_exact_add(const double* a, const double* b, double* out, int64_t
 int nd_selftest_exact_scan(const double* terms, const int64_t* seg, const double* s0, double* out, int64_t nseg,
                            void* stream);
 
+/* out[i] = a[i] / b[i] with the integer binary64 division of the FP64 kernels. */
+int nd_selftest_exact_div(const double* a, const double* b, double* out, int64_t n, void* stream);
+
 /* s[i] = sin x[i], c[i] = cos x[i] with the fixed-point functions of the FP64 kernels. */
 int nd_selftest_trig(const double* x, double* s, double* c, int64_t n, void* stream);
 

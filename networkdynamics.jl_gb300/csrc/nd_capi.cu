@@ -683,6 +683,13 @@ int nd_selftest_exact_add(const double* a, const double* b, double* out, int64_t
     return err == cudaSuccess ? ND_OK : cuda_fail(err, "nd_selftest_exact_add");
 }
 
+int nd_selftest_exact_div(const double* a, const double* b, double* out, int64_t n, void* stream) {
+    clear_error();
+    if (n < 0 || (n > 0 && (!a || !b || !out))) return fail(ND_ERR_ARG, "nd_selftest_exact_div: bad arguments");
+    cudaError_t err = launch_div_selftest(a, b, out, n, (cudaStream_t)stream);
+    return err == cudaSuccess ? ND_OK : cuda_fail(err, "nd_selftest_exact_div");
+}
+
 int nd_selftest_trig(const double* x, double* s, double* c, int64_t n, void* stream) {
     clear_error();
     if (n < 0 || (n > 0 && (!x || !s || !c))) return fail(ND_ERR_ARG, "nd_selftest_trig: bad arguments");

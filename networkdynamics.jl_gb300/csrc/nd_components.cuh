@@ -19,11 +19,14 @@ struct Arith<double> {
     static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
     static __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
     static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
-    static __device__ __forceinline__ double div(double a, double b) { return __ddiv_rn(a, b); }
+    static __device__ __forceinline__ double div(double a, double b) { return exact::div_rn(a, b); }
     // FP64 keeps the raw phase difference, like the reference's sin(θs - θd); both functions
     // run on the integer pipes (nd_trig.cuh).
     static __device__ __forceinline__ double sin_phase(double x) { return trig::sin(x); }
     static __device__ __forceinline__ double cos_phase(double x) { return trig::cos(x); }
+    // w sin(x) and w cos(x)
+    static __device__ __forceinline__ double times_sin(double w, double x) { return trig::times_sin(w, x); }
+    static __device__ __forceinline__ double times_cos(double w, double x) { return trig::times_cos(w, x); }
 };
 
 // 2π split for a two-step Cody–Waite reduction of a phase difference to [-π, π].
@@ -50,6 +53,8 @@ struct Arith<float> {
     }
     static __device__ __forceinline__ float sin_phase(float x) { return sinf(wrap(x)); }
     static __device__ __forceinline__ float cos_phase(float x) { return cosf(wrap(x)); }
+    static __device__ __forceinline__ float times_sin(float w, float x) { return mul(w, sin_phase(x)); }
+    static __device__ __forceinline__ float times_cos(float w, float x) { return mul(w, cos_phase(x)); }
 };
 
 // Read-only load of a component parameter (a plain read for value types that are not
@@ -68,7 +73,7 @@ __device__ __forceinline__ T edge_g(T vs, T vd, const T* __restrict__ pe, int32_
     } else if constexpr (EK == ND_E_DIFFUSION_UNIT) {
         return A::sub(vs, vd);                         // e .= v_s .- v_d
     } else {
-        return A::mul(__ldg(pe + e), A::sin_phase(A::sub(vs, vd)));  // e .= K .* sin(θs - θd)
+        return A::times_sin(__ldg(pe + e), A::sub(vs, vd));  // e .= K .* sin(θs - θd)
     }
 }
 
@@ -82,7 +87,7 @@ __device__ __forceinline__ T edge_g_w(T vs, T vd, T w) {
     } else if constexpr (EK == ND_E_DIFFUSION_UNIT) {
         return A::sub(vs, vd);
     } else {
-        return A::mul(w, A::sin_phase(A::sub(vs, vd)));
+        return A::times_sin(w, A::sub(vs, vd));
     }
 }
 

@@ -145,7 +145,7 @@ __device__ void instance_rhs(const EnsArgs& a, const Inst& s, const TU* __restri
                 T term;
                 if constexpr (EK == ND_E_DIFFUSION) term = A::mul(pe[e], d);
                 else if constexpr (EK == ND_E_DIFFUSION_UNIT) term = d;
-                else term = A::mul(pe[e], A::sin_phase(d));
+                else term = A::times_sin(pe[e], d);
                 acc = A::add(acc, term);
             }
         } else {
@@ -234,16 +234,38 @@ __global__ void ens_rhs_kernel(EnsArgs a, const typename Elem<T>::type* __restri
     }
 }
 
-__device__ __forceinline__ double block_sum(double v, double* red) {
+// Fixed-order block sums of NS values at once, the same in every thread.  The threads' values go
+// through shared memory and one warp adds each of the sums: a butterfly in every warp (5 FP64
+// adds each) and the warps' totals in every thread took a fifth of the Newton kernel's FP64 time.
+constexpr int kMaxThreads = 512;
+template <int NS>
+struct BlockSums {
+    double val[NS][kMaxThreads];
+    double sum[NS];
+};
+template <int NS>
+__device__ __forceinline__ void block_sums(double (&v)[NS], BlockSums<NS>& sh) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncthreads();  // sums of the call before are read
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFullMask, v, off);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int k = 0; k < NS; ++k) sh.val[k][threadIdx.x] = v[k];
     __syncthreads();
-    if (lane == 0) red[w] = v;
+    if (w < NS) {  // blocks have at least two warps
+        double t = 0.0;
+        for (int j = lane; j < (int)blockDim.x; j += 32) t += sh.val[w][j];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(kFullMask, t, off);
+        if (lane == 0) sh.sum[w] = t;
+    }
     __syncthreads();
-    double t = 0.0;
-    for (int k = 0; k < nw; ++k) t += red[k];  // fixed order: deterministic
-    return t;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) v[k] = sh.sum[k];
+}
+template <int NS>
+__device__ __forceinline__ double block_sum(double v, BlockSums<NS>& sh) {
+    double t[NS] = {v};
+    block_sums<NS>(t, sh);
+    return t[0];
 }
 
 __device__ __forceinline__ int take_instance(const EnsArgs& a, int* sh) {
@@ -251,6 +273,12 @@ __device__ __forceinline__ int take_instance(const EnsArgs& a, int* sh) {
     if (threadIdx.x == 0) *sh = atomicAdd(a.counter, 1);
     __syncthreads();
     return *sh;
+}
+
+// max(|a|, |b|) without the FP64 unit (NaN wins, so that it reaches the error norm)
+__device__ __forceinline__ double max_abs(double a, double b) {
+    const uint64_t x = exact::to_bits(a) & ~exact::kSign, y = exact::to_bits(b) & ~exact::kSign;
+    return exact::from_bits(x > y ? x : y);
 }
 
 // ---- batched Tsit5 ----------------------------------------------------------------------
@@ -265,10 +293,11 @@ struct SolveParams {
 };
 
 template <typename T, int VK, int EK>
-__global__ void ens_tsit5_kernel(EnsArgs a, SolveParams sp, double* __restrict__ U,
+__global__ void __launch_bounds__(kMaxThreads) ens_tsit5_kernel(EnsArgs a, SolveParams sp, double* __restrict__ U,
                                  const typename Elem<T>::type* __restrict__ p,
                                  double* __restrict__ work, int32_t* __restrict__ status, int64_t* __restrict__ nsteps) {
-    __shared__ double red[32];
+    using A = Arith<double>;
+    __shared__ BlockSums<2> red;
     __shared__ int sh_inst;
     __shared__ double sh_dt, sh_t, sh_qold;
     __shared__ int sh_accept, sh_done, sh_status;
@@ -287,15 +316,15 @@ __global__ void ens_tsit5_kernel(EnsArgs a, SolveParams sp, double* __restrict__
         // k0 = f(u); initial step (Hairer & Wanner)
         any_instance_rhs<T, VK, EK>(a, s, U, p, K[0]);
         __syncthreads();
-        double d0 = 0, d1 = 0;
+        double d01[2] = {0.0, 0.0};
         for (int64_t j = threadIdx.x; j < n; j += blockDim.x) {
             const double sc = sp.abstol + fabs(u[j]) * sp.reltol;
-            d0 += (u[j] / sc) * (u[j] / sc);
-            d1 += (K[0][s.ubase + j] / sc) * (K[0][s.ubase + j] / sc);
+            const double r0 = A::div(u[j], sc), r1 = A::div(K[0][s.ubase + j], sc);
+            d01[0] += r0 * r0;
+            d01[1] += r1 * r1;
         }
-        d0 = sqrt(block_sum(d0, red) / (double)(n ? n : 1));
-        __syncthreads();
-        d1 = sqrt(block_sum(d1, red) / (double)(n ? n : 1));
+        block_sums<2>(d01, red);
+        const double d0 = sqrt(d01[0] / (double)(n ? n : 1)), d1 = sqrt(d01[1] / (double)(n ? n : 1));
         double h0 = (d0 < 1e-5 || d1 < 1e-5) ? 1e-6 : 0.01 * (d0 / d1);
         h0 = fmin(h0, sp.t1 - sp.t0);
         for (int64_t j = threadIdx.x; j < n; j += blockDim.x) Y[s.ubase + j] = u[j] + h0 * K[0][s.ubase + j];
@@ -305,10 +334,9 @@ __global__ void ens_tsit5_kernel(EnsArgs a, SolveParams sp, double* __restrict__
         double d2 = 0;
         for (int64_t j = threadIdx.x; j < n; j += blockDim.x) {
             const double sc = sp.abstol + fabs(u[j]) * sp.reltol;
-            const double r = (K[1][s.ubase + j] - K[0][s.ubase + j]) / sc;
+            const double r = A::div(K[1][s.ubase + j] - K[0][s.ubase + j], sc);
             d2 += r * r;
         }
-        __syncthreads();
         d2 = sqrt(block_sum(d2, red) / (double)(n ? n : 1)) / h0;
         if (threadIdx.x == 0) {
             const double h1 = (fmax(d1, d2) <= 1e-15) ? fmax(1e-6, h0 * 1e-3) : pow(0.01 / fmax(d1, d2), 1.0 / 5.0);
@@ -327,24 +355,39 @@ __global__ void ens_tsit5_kernel(EnsArgs a, SolveParams sp, double* __restrict__
         __syncthreads();
         while (!sh_done) {
             const double h = sh_dt;
-            for (int st = 1; st < 7; ++st) {
+            // y = u + h Σ_j a_j k_j by fused multiply-adds, the sum first: only the last one rounds
+            // at the size of u
+            auto stage = [&](auto ic) {
+                constexpr int st = decltype(ic)::value;
+#pragma unroll 2
                 for (int64_t j = threadIdx.x; j < n; j += blockDim.x) {
-                    double acc = 0.0;
-                    for (int m = 0; m < st; ++m) acc = __dadd_rn(acc, __dmul_rn(e_a[st][m], K[m][s.ubase + j]));
-                    Y[s.ubase + j] = __dadd_rn(u[j], __dmul_rn(h, acc));
+                    double d = __dmul_rn(e_a[st][0], K[0][s.ubase + j]);
+#pragma unroll
+                    for (int m = 1; m < st; ++m) d = __fma_rn(e_a[st][m], K[m][s.ubase + j], d);
+                    Y[s.ubase + j] = __fma_rn(h, d, u[j]);
                 }
                 __syncthreads();
                 any_instance_rhs<T, VK, EK>(a, s, Y, p, K[st]);
                 __syncthreads();
-            }
+            };
+            stage(std::integral_constant<int, 1>{});
+            stage(std::integral_constant<int, 2>{});
+            stage(std::integral_constant<int, 3>{});
+            stage(std::integral_constant<int, 4>{});
+            stage(std::integral_constant<int, 5>{});
+            stage(std::integral_constant<int, 6>{});
             double se = 0.0;
+#pragma unroll 2
             for (int64_t j = threadIdx.x; j < n; j += blockDim.x) {
-                double acc = 0.0;
-                for (int m = 0; m < 7; ++m) acc = __dadd_rn(acc, __dmul_rn(e_bt[m], K[m][s.ubase + j]));
-                const double e = __dmul_rn(h, acc);
-                const double sc = sp.abstol + sp.reltol * fmax(fabs(u[j]), fabs(Y[s.ubase + j]));
-                const double r = e / sc;
-                se += r * r;
+                // the weights sum to zero, so they enter as they are: h times a weight, rounded,
+                // would shift the estimate of all entries together
+                double e = __dmul_rn(e_bt[0], K[0][s.ubase + j]);
+#pragma unroll
+                for (int m = 1; m < 7; ++m) e = __fma_rn(e_bt[m], K[m][s.ubase + j], e);
+                e = __dmul_rn(h, e);
+                const double sc = __fma_rn(sp.reltol, max_abs(u[j], Y[s.ubase + j]), sp.abstol);
+                const double r = A::div(e, sc);
+                se = __fma_rn(r, r, se);
             }
             const double tot = block_sum(se, red);
             if (threadIdx.x == 0) {
@@ -401,8 +444,11 @@ __global__ void ens_tsit5_kernel(EnsArgs a, SolveParams sp, double* __restrict__
 // ---- batched Newton-CG for swing steady states ------------------------------------------------
 // Reduced system at ω = 0: G_v(θ) = Pm_v + Σ_e (K sin terms of the edges at v), exactly
 // the aggregation of the RHS.  -∂G/∂θ is the weighted Laplacian with w = K cos(θ_n - θ_v);
-// each Newton step solves -J δ = G by CG in the subspace orthogonal to the uniform phase
-// shift (G and every Laplacian image are orthogonal to it).
+// each Newton step solves -J δ = G by CG, preconditioned by the diagonal Σ |w| (hubs of a
+// scale-free network spread the diagonal over two orders of magnitude: 306 iterations a
+// solve without it on BA(2000, 2), 106 with it).  G and every Laplacian image are orthogonal to
+// the uniform phase shift; the shift itself, which the preconditioner lets into the solution, is
+// free and taken out at the end.
 struct NewtonParams {
     double tol;
     int max_newton, max_cg;
@@ -415,14 +461,16 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
                                   double* __restrict__ work, int32_t* __restrict__ iters, double* __restrict__ resid,
                                   int32_t* __restrict__ status, int32_t* __restrict__ cg_total) {
     using A = Arith<double>;
-    __shared__ double red[32];
+    __shared__ BlockSums<2> red;
+    __shared__ double wmax[32];
     __shared__ int sh_inst;
     double* X = work;               // Newton step / CG solution
     double* R = work + np.nv;       // CG residual
     double* Pd = work + 2 * np.nv;  // CG direction
     double* Q = work + 3 * np.nv;   // -J · direction
     double* G = work + 4 * np.nv;   // power mismatch
-    double* W = work + 5 * np.nv;   // [ninc] incidence weights K cos(θ_n - θ_v)
+    double* Di = work + 5 * np.nv;  // 1 / Σ |w|
+    double* W = work + 6 * np.nv;   // [ninc] incidence weights K cos(θ_n - θ_v)
     for (;;) {
         const int q = take_instance(a, &sh_inst);
         if (q >= a.n_inst) break;
@@ -451,10 +499,10 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(kFullMask, mx, off));
             __syncthreads();
-            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+            if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mx;
             __syncthreads();
             res = 0.0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) res = fmax(res, red[w]);
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) res = fmax(res, wmax[w]);
             __syncthreads();
             if (res <= np.tol) break;
             if (!(res == res)) {
@@ -465,41 +513,41 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
                 st = ND_ERR_MAXITERS;
                 break;
             }
-            // weights and CG init: X = 0, R = G, P = R
+            // weights, preconditioner and CG start: X = 0, R = G without its mean.  The right-hand
+            // side is kept orthogonal to the uniform shift (it is, up to rounding): a component
+            // along the null space would make CG grow x without bound along it.
+            double gm = 0.0;
+            for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) gm += G[s.vbase + v];
+            gm = block_sum(gm, red) / (double)nvi;
+            double rs[2] = {0.0, 0.0};  // r · r, r · z
             for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) {
                 const uint32_t beg = a.row_ptr[s.vbase + v], end = a.row_ptr[s.vbase + v + 1];
                 const double uv = th[2 * v];
+                double d = 0.0;
                 for (uint32_t k = beg; k < end; ++k) {
                     const int32_t eb = a.eid[k];
                     const double Kk = EK == ND_E_DIFFUSION_UNIT ? 1.0 : pe[eb & 0x7fffffff];
                     const double dth = th[2 * (int64_t)a.nbr[k]] - uv;
-                    W[k] = EK == ND_E_KURAMOTO ? Kk * A::cos_phase(dth) : Kk;
+                    W[k] = EK == ND_E_KURAMOTO ? A::times_cos(Kk, dth) : Kk;
+                    d += fabs(W[k]);
                 }
+                const double di = d > 0.0 ? A::div(1.0, d) : 1.0;
+                const double r = G[s.vbase + v] - gm, z = di * r;
+                Di[s.vbase + v] = di;
                 X[s.vbase + v] = 0.0;
-                R[s.vbase + v] = G[s.vbase + v];
-                Pd[s.vbase + v] = G[s.vbase + v];
+                R[s.vbase + v] = r;
+                Pd[s.vbase + v] = z;
+                rs[0] += r * r;
+                rs[1] += r * z;
             }
-            __syncthreads();
-            // keep the right-hand side orthogonal to the uniform shift (it is, up to rounding):
-            // a component along the null space would make CG grow x without bound along it
-            double gm = 0.0;
-            for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) gm += R[s.vbase + v];
-            gm = block_sum(gm, red) / (double)nvi;
-            for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) {
-                R[s.vbase + v] -= gm;
-                Pd[s.vbase + v] -= gm;
-            }
-            __syncthreads();
-            double rr = 0.0;
-            for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) rr += R[s.vbase + v] * R[s.vbase + v];
-            rr = block_sum(rr, red);
-            const double rr0 = rr;
+            block_sums<2>(rs, red);  // its barriers also publish W and Pd
+            double rz = rs[1];
+            const double rr0 = rs[0];
             // stop at a relative residual of cg_rtol, or once the linear residual is far
             // below the Newton tolerance
             const double floor2 = (1e-3 * np.tol) * (1e-3 * np.tol);
             int cg = 0;
-            while (cg < np.max_cg && rr > np.cg_rtol * np.cg_rtol * rr0 && rr > floor2) {
-                __syncthreads();
+            while (cg < np.max_cg && rs[0] > np.cg_rtol * np.cg_rtol * rr0 && rs[0] > floor2) {
                 double pq = 0.0;
                 for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) {
                     const uint32_t beg = a.row_ptr[s.vbase + v], end = a.row_ptr[s.vbase + v + 1];
@@ -510,18 +558,21 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
                     pq += pvv * acc;
                 }
                 pq = block_sum(pq, red);
-                const double alpha = rr / pq;
-                double rr_new = 0.0;
+                const double alpha = rz / pq;
+                rs[0] = rs[1] = 0.0;
                 for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) {
                     X[s.vbase + v] += alpha * Pd[s.vbase + v];
-                    R[s.vbase + v] -= alpha * Q[s.vbase + v];
-                    rr_new += R[s.vbase + v] * R[s.vbase + v];
+                    const double r = R[s.vbase + v] - alpha * Q[s.vbase + v];
+                    R[s.vbase + v] = r;
+                    rs[0] += r * r;
+                    rs[1] += r * (Di[s.vbase + v] * r);
                 }
-                rr_new = block_sum(rr_new, red);
-                const double beta = rr_new / rr;
-                rr = rr_new;
+                block_sums<2>(rs, red);
+                const double beta = rs[1] / rz;
+                rz = rs[1];
                 for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x)
-                    Pd[s.vbase + v] = R[s.vbase + v] + beta * Pd[s.vbase + v];
+                    Pd[s.vbase + v] = Di[s.vbase + v] * R[s.vbase + v] + beta * Pd[s.vbase + v];
+                __syncthreads();
                 ++cg;
             }
             cgsum += cg;
@@ -604,6 +655,16 @@ EnsArgs args_of(nd_ensemble* e) {
     a.eid = e->incid_eid;
     a.counter = e->counter;
     return a;
+}
+
+// Threads per instance when neither the caller nor the autotuner chose: one to two rows of an
+// average instance per thread, within 64 to 512.  More threads than rows idle; fewer leave the
+// largest instances running alone at the end, because an SM then holds so many blocks that
+// every instance starts at once and nothing is left in the queue to balance: 1024 instances of
+// 50 to 2000 vertices took 160, 97, 60 and 60 ms with 64, 128, 256 and 512 threads.
+int default_threads(const nd_ensemble* e) {
+    const int64_t rows = e->nv / e->n_inst;
+    return rows >= 512 ? 512 : (rows >= 256 ? 256 : (rows >= 128 ? 128 : 64));
 }
 
 cudaError_t ensure_work(nd_ensemble* e, size_t bytes) {
@@ -760,7 +821,7 @@ int nd_ensemble_solve_tsit5_ex(nd_ensemble* e, double* u, const void* p, double 
     if (!e || !u || !status || !nsteps) return fail(ND_ERR_ARG, "nd_ensemble_solve_tsit5: NULL argument");
     if (!(t1 > t0) || !(reltol > 0) || !(abstol > 0)) return fail(ND_ERR_ARG, "nd_ensemble_solve_tsit5: bad time span or tolerances");
     if (e->pdim > 0 && !p) return fail(ND_ERR_ARG, "nd_ensemble_solve_tsit5: p is NULL");
-    if (threads == 0) threads = e->tuned_threads ? e->tuned_threads : 128;
+    if (threads == 0) threads = e->tuned_threads ? e->tuned_threads : default_threads(e);
     if (threads != 64 && threads != 128 && threads != 256 && threads != 512)
         return fail(ND_ERR_ARG, "nd_ensemble_solve_tsit5: threads must be 64, 128, 256 or 512 (0 = tuned)");
     cudaError_t err = upload_tableau();
@@ -828,7 +889,7 @@ int nd_ensemble_fixpoint(nd_ensemble* e, double* u, const double* p, double tol,
     if (e->dtype != ND_F64) return fail(ND_ERR_DTYPE, "nd_ensemble_fixpoint: the Newton solve runs in FP64");
     if (!(tol > 0) || max_newton <= 0) return fail(ND_ERR_ARG, "nd_ensemble_fixpoint: bad tolerance or budget");
     if (max_cg <= 0) max_cg = std::max(100, 4 * e->max_rows);
-    cudaError_t err = ensure_work(e, sizeof(double) * ((size_t)5 * e->nv + (size_t)2 * e->ne + 1));
+    cudaError_t err = ensure_work(e, sizeof(double) * ((size_t)6 * e->nv + (size_t)2 * e->ne + 1));
     if (err != cudaSuccess) return cuda_fail(err, "workspace");
     cudaStream_t s = (cudaStream_t)stream;
     if ((err = cudaMemsetAsync(e->counter, 0, sizeof(int), s)) != cudaSuccess) return cuda_fail(err, "memset");

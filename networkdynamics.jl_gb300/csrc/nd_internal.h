@@ -324,6 +324,7 @@ struct GmresSolver {
 void vec_axpby(int64_t n, double a, const double* x, double b, double* y, cudaStream_t s);  // y = a x + b y
 
 cudaError_t launch_exact_selftest(const double* a, const double* b, double* out, int64_t n, cudaStream_t s);
+cudaError_t launch_div_selftest(const double* a, const double* b, double* out, int64_t n, cudaStream_t s);
 cudaError_t launch_trig_selftest(const double* x, double* s, double* c, int64_t n, cudaStream_t st);
 cudaError_t launch_scan_selftest(const double* terms, const int64_t* seg, const double* s0, double* out,
                                  int64_t nseg, cudaStream_t s);

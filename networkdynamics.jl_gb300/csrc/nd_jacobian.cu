@@ -94,7 +94,7 @@ __device__ __forceinline__ void static_edge_dg(int kind, T vs, T vd, T w, T& gs,
         gs = T(1);
         gd = T(-1);
     } else {
-        const T c = A::mul(w, A::cos_phase(A::sub(vs, vd)));  // K cos(θs - θd)
+        const T c = A::times_cos(w, A::sub(vs, vd));  // K cos(θs - θd)
         gs = c;
         gd = -c;
     }

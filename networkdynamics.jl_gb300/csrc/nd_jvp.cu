@@ -33,7 +33,7 @@ __device__ __forceinline__ T jvp_term(int2 inc, T uv, T dv, const T* __restrict_
     T c;
     if constexpr (EK == ND_E_DIFFUSION) c = pe[e];
     else if constexpr (EK == ND_E_DIFFUSION_UNIT) c = T(1);
-    else c = A::mul(pe[e], A::cos_phase(A::sub(u[n * DV], uv)));
+    else c = A::times_cos(pe[e], A::sub(u[n * DV], uv));
     return A::mul(c, A::sub(vv[n * DV], dv));
 }
 

@@ -343,6 +343,12 @@ __global__ void exact_add_selftest_kernel(const double* a, const double* b, doub
     if (i < n) out[i] = exact::add_rn(a[i], b[i]);
 }
 
+// Self-test of the integer division.
+__global__ void exact_div_selftest_kernel(const double* a, const double* b, double* out, int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = exact::div_rn(a[i], b[i]);
+}
+
 // Self-test of the fixed-point sine and cosine.
 __global__ void trig_selftest_kernel(const double* x, double* s, double* c, int64_t n) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -400,6 +406,12 @@ cudaError_t launch_rhs(int dtype, const RhsArgs& a, cudaStream_t s) {
 cudaError_t launch_exact_selftest(const double* a, const double* b, double* out, int64_t n, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     exact_add_selftest_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, b, out, n);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_div_selftest(const double* a, const double* b, double* out, int64_t n, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    exact_div_selftest_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, b, out, n);
     return cudaGetLastError();
 }
 

@@ -1,5 +1,6 @@
-"""The fixed-point sine and cosine of the FP64 kernels (networkdynamics.jl_gb300/csrc/nd_trig.cuh)
-against extended precision on the host, and the device build against the host build, bit for bit."""
+"""The fixed-point sine and cosine (networkdynamics.jl_gb300/csrc/nd_trig.cuh) and the integer
+division (nd_exact.cuh) of the FP64 kernels against extended precision and IEEE-754 division on the
+host, and the device build against the host build, bit for bit."""
 import ctypes as C
 import subprocess
 from pathlib import Path
@@ -23,13 +24,58 @@ def host():
                         "-o", str(out)], check=True)
     lib = C.CDLL(str(out))
     lib.nd_trig_host.argtypes = [C.c_void_p] * 3 + [C.c_int64]
+    lib.nd_trig_times_host.argtypes = [C.c_void_p] * 4 + [C.c_int64]
+    lib.nd_exact_div_host.argtypes = [C.c_void_p] * 3 + [C.c_int64]
 
-    def run(x):
+    def run(x, f=None):
         x = np.ascontiguousarray(x, dtype=np.float64)
         s, c = np.empty_like(x), np.empty_like(x)
-        lib.nd_trig_host(x.ctypes.data, s.ctypes.data, c.ctypes.data, x.size)
+        if f is None:
+            lib.nd_trig_host(x.ctypes.data, s.ctypes.data, c.ctypes.data, x.size)
+        else:
+            lib.nd_trig_times_host(f.ctypes.data, x.ctypes.data, s.ctypes.data, c.ctypes.data, x.size)
         return s, c
+
+    def div(a, b):
+        out = np.empty_like(a)
+        lib.nd_exact_div_host(a.ctypes.data, b.ctypes.data, out.ctypes.data, a.size)
+        return out
+    run.div = div
     return run
+
+
+def factors(n, seed):
+    """Line weights of every size, zeros and the ends of the exponent range."""
+    rng = np.random.default_rng(seed)
+    f = rng.uniform(5, 10, n) * 10.0 ** rng.choice([0, 0, 0, -5, 5], n) * rng.choice([1.0, -1.0], n)
+    f[:8] = [0.0, -0.0, 5e-324, 1e-300, 1e308, np.inf, np.nan, 1.0]
+    return f
+
+
+def quotients(n, seed):
+    """Operands of ordinary size, any bit pattern, powers of two, and quotients next to a
+    halfway point (a = RN(b (q + 1/2 ulp)))."""
+    rng = np.random.default_rng(seed)
+    bits = lambda: rng.integers(0, 2 ** 64, n, dtype=np.uint64).view(np.float64)  # noqa: E731
+    b, q = rng.uniform(0.5, 2, n), rng.uniform(0.5, 2, n)
+    yield rng.normal(size=n), rng.normal(size=n) * 10.0 ** rng.integers(-20, 20, n)
+    yield bits(), bits()
+    yield np.ones(n), rng.integers(1, 1 << 53, n).astype(np.float64)
+    yield 2.0 ** rng.integers(-1074, 1024, n), 2.0 ** rng.integers(-1074, 1024, n)
+    yield (b.astype(np.longdouble) * (q.astype(np.longdouble) + np.spacing(q) / 2)).astype(np.float64), b
+    z = np.array([0.0, -0.0, 1.0, -1.0, np.inf, -np.inf, np.nan, 5e-324, 1.7976931348623157e308, 2.2250738585072014e-308])
+    a, b = np.meshgrid(z, z)
+    yield a.ravel().copy(), b.ravel().copy()
+
+
+def same_bits(a, b):
+    return np.all((a.view(np.uint64) == b.view(np.uint64)) | (np.isnan(a) & np.isnan(b)))
+
+
+def test_host_division_matches_ieee(host):
+    with np.errstate(all="ignore"):
+        for a, b in quotients(400_000, 3):
+            assert same_bits(host.div(a, b), a / b)
 
 
 def arguments(n, seed=0):
@@ -56,6 +102,16 @@ def test_host_error_below_051_ulp(host):
     for got, ref in ((s, np.sin(xl)), (c, np.cos(xl))):
         ulp = np.spacing(np.abs(ref.astype(np.float64)))
         assert float(np.max(np.abs(got.astype(np.longdouble) - ref) / ulp)) <= 0.51
+    # the products: once more 2^-61 (the library's and tiny arguments take the plain product)
+    f = factors(x.size, 1)[8:]
+    x = x[8:]
+    xl, fl = x.astype(np.longdouble), f.astype(np.longdouble)
+    half_pi = np.longdouble("1.5707963267948966192313216916397514421")
+    k = np.rint(xl / half_pi)
+    plain = (np.abs(x) >= 2.0 ** 17) | (np.abs(x) < 2.0 ** -27) | ((np.abs(xl - k * half_pi) < 2.0 ** -17) & (k != 0))
+    for got, ref in zip(host(x, f), (fl * np.sin(xl), fl * np.cos(xl))):
+        err = np.abs(got.astype(np.longdouble) - ref) / np.spacing(np.abs(ref.astype(np.float64)))
+        assert float(np.max(err[~plain])) <= 0.51
 
 
 def test_host_symmetry_and_special_values(host):
@@ -63,6 +119,10 @@ def test_host_symmetry_and_special_values(host):
     s, c = host(x)
     sn, cn = host(-x)
     assert np.array_equal(sn, -s) and np.array_equal(cn, c)
+    f = factors(x.size, 2)
+    with np.errstate(all="ignore"):
+        for got, ref in zip(host(x[:8], f[:8].copy()), (f[:8] * np.sin(x[:8]), f[:8] * np.cos(x[:8]))):
+            np.testing.assert_allclose(got, ref, rtol=2.0 ** -51, atol=5e-324)
     s, c = host([0.0, -0.0, 5e-324, -2.0 ** -1030, np.inf, -np.inf, np.nan])
     assert np.array_equal(s[:4], [0.0, -0.0, 5e-324, -2.0 ** -1030]) and np.signbit(s[1]) and not np.signbit(s[0])
     assert np.array_equal(c[:4], np.ones(4)) and np.isnan(s[4:]).all() and np.isnan(c[4:]).all()
@@ -86,6 +146,13 @@ def test_device_matches_host(host, cuda):
     for got, ref in zip((st.cpu().numpy(), ct.cpu().numpy()), host(x)):
         np.testing.assert_array_equal(got[~library], ref[~library])
         assert np.all(np.abs(got - ref)[library] <= 2 * np.spacing(np.abs(ref[library])))
+    for a, b in quotients(400_000, 4):
+        at, bt = torch.from_numpy(a).to(cuda), torch.from_numpy(b).to(cuda)
+        qt = torch.empty_like(at)
+        capi.check(lib.nd_selftest_exact_div(at.data_ptr(), bt.data_ptr(), qt.data_ptr(), a.size,
+                                             C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        with np.errstate(all="ignore"):
+            assert same_bits(qt.cpu().numpy(), a / b)
     sm = torch.empty_like(xt)
     capi.check(lib.nd_selftest_trig((-xt).data_ptr(), sm.data_ptr(), ct.data_ptr(), x.size,
                                     C.c_void_p(torch.cuda.current_stream().cuda_stream)))
