@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kBlock, 8) rhs_kernel(RhsArgs a) {
 // serial, and on a crowded SM each of its steps waits for other blocks' instructions.
 constexpr int kHeavySoloSmem = 160 * 1024;
 
-// FP64 sequential sum of a heavy row by one block: tiles of kBlockTile terms, each added by the
+// FP64 sequential sum of a heavy row by one block: tiles of kScanTile terms, each added by the
 // block-wide exact scan (or the hardware DADD chain in the native mode).  A thread's incidence
 // data of the next tile are in flight while the current tile is added.
 template <int VK, int EK, int MODE>
@@ -218,11 +218,11 @@ __device__ __forceinline__ void solo_row_fp64(const RhsArgs& a, int slot, double
     const int tid = threadIdx.x;
     double un[kBlockPer], w[kBlockPer];
     unsigned src_side = 0;
-    auto load = [&](uint32_t base) {  // positions tid, tid + kBlock, ...: coalesced
+    auto load = [&](uint32_t base) {  // positions tid, tid + kScanThreads, ...: coalesced
         src_side = 0;
 #pragma unroll
         for (int k = 0; k < kBlockPer; ++k) {
-            const uint32_t i = base + (uint32_t)(tid + k * kBlock);
+            const uint32_t i = base + (uint32_t)(tid + k * kScanThreads);
             un[k] = w[k] = 0.0;
             if (i < end) {
                 const int2 inc = ld_hint(incid + i, stream);
@@ -234,14 +234,14 @@ __device__ __forceinline__ void solo_row_fp64(const RhsArgs& a, int slot, double
     };
     load(beg);
     double S = 0.0;
-    for (uint32_t base = beg; base < end; base += kBlockTile) {
-        const int n = (int)min((uint32_t)kBlockTile, end - base);
+    for (uint32_t base = beg; base < end; base += kScanTile) {
+        const int n = (int)min((uint32_t)kScanTile, end - base);
 #pragma unroll
         for (int k = 0; k < kBlockPer; ++k)
-            if (tid + k * kBlock < n)
-                tile[tile_at(tid + k * kBlock)] = incidence_term_w<double, EK>(uv, un[k], w[k], (src_side >> k) & 1u);
+            if (tid + k * kScanThreads < n)
+                tile[tile_at(tid + k * kScanThreads)] = incidence_term_w<double, EK>(uv, un[k], w[k], (src_side >> k) & 1u);
         __syncthreads();
-        load(base + kBlockTile);
+        load(base + kScanTile);
         if constexpr (MODE == kModeNative) {
             if (tid < 32)
                 for (int i = 0; i < n; ++i) S = __dadd_rn(S, tile[tile_at(i)]);
@@ -256,7 +256,7 @@ __device__ __forceinline__ void solo_row_fp64(const RhsArgs& a, int slot, double
 template <typename T, int VK, int EK, int MODE>
 __global__ void __launch_bounds__(kBlock, 1) heavy_solo_kernel(RhsArgs a) {
     if constexpr (sizeof(T) == 8 && MODE != kModeTree) {
-        __shared__ double tile[kBlockTilePadded];
+        __shared__ double tile[kScanTilePadded];
         __shared__ BlockScanShared sh;
         solo_row_fp64<VK, EK, MODE>(a, blockIdx.x, tile, sh);
     } else {
@@ -265,12 +265,13 @@ __global__ void __launch_bounds__(kBlock, 1) heavy_solo_kernel(RhsArgs a) {
     }
 }
 
-// The FP64 sequential rows ask for 18 KB of shared memory, so that a block also fits on an SM
-// that holds several edge-phase blocks; they run on the handle's high-priority side stream.
+// The FP64 sequential rows ask for 15 KB of shared memory and 128 threads, so that a block also
+// fits on an SM that holds several edge-phase blocks; they run on the handle's high-priority side stream.
 // The FP32 and tree rows ask for most of an SM (kHeavySoloSmem).
 template <typename T, int VK, int EK, int MODE>
 cudaError_t launch_heavy_solo(const RhsArgs& a, cudaStream_t s) {
-    constexpr int smem = sizeof(T) == 8 && MODE != kModeTree ? 0 : kHeavySoloSmem;
+    constexpr bool scan = sizeof(T) == 8 && MODE != kModeTree;
+    constexpr int smem = scan ? 0 : kHeavySoloSmem;
     if constexpr (smem > 0) {
         static int attr_set = 0;  // per instantiation; the attribute is per function
         if (attr_set < smem) {
@@ -280,7 +281,7 @@ cudaError_t launch_heavy_solo(const RhsArgs& a, cudaStream_t s) {
             attr_set = smem;
         }
     }
-    heavy_solo_kernel<T, VK, EK, MODE><<<a.n_heavy, kBlock, smem, s>>>(a);
+    heavy_solo_kernel<T, VK, EK, MODE><<<a.n_heavy, scan ? kScanThreads : kBlock, smem, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -363,7 +364,7 @@ __global__ void trig_selftest_kernel(const double* x, double* s, double* c, int6
 // the sliding 256-term scan (w % 8 == 0) or the block-wide scan of the heavy rows (w % 8 == 4).
 __global__ void exact_scan_selftest_kernel(const double* terms, const int64_t* seg, const double* s0, double* out,
                                            int64_t nseg) {
-    __shared__ double tile[kBlockTilePadded];
+    __shared__ double tile[kTile];  // kScanTilePadded entries or more
     __shared__ BlockScanShared sh;
     const int64_t w = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -378,8 +379,8 @@ __global__ void exact_scan_selftest_kernel(const double* terms, const int64_t* s
             }
         }
     } else if ((w & 7) == 4) {
-        for (int64_t base = seg[w]; base < seg[w + 1]; base += kBlockTile) {
-            const int n = (int)min((int64_t)kBlockTile, seg[w + 1] - base);
+        for (int64_t base = seg[w]; base < seg[w + 1]; base += kScanTile) {
+            const int n = (int)min((int64_t)kScanTile, seg[w + 1] - base);
             for (int i = threadIdx.x; i < n; i += blockDim.x) tile[tile_at(i)] = terms[base + i];
             __syncthreads();
             S = exact_scan_block(S, tile, n, sh);
@@ -424,7 +425,7 @@ cudaError_t launch_trig_selftest(const double* x, double* s, double* c, int64_t 
 cudaError_t launch_scan_selftest(const double* terms, const int64_t* seg, const double* s0, double* out, int64_t nseg,
                                  cudaStream_t s) {
     if (nseg <= 0) return cudaSuccess;
-    exact_scan_selftest_kernel<<<(unsigned)nseg, kBlock, 0, s>>>(terms, seg, s0, out, nseg);
+    exact_scan_selftest_kernel<<<(unsigned)nseg, kScanThreads, 0, s>>>(terms, seg, s0, out, nseg);
     return cudaGetLastError();
 }
 

@@ -344,78 +344,79 @@ static __device__ __forceinline__ double exact_scan_wide(double S, const double*
 // A long row is one chain of dependent roundings: 63 clocks a term with hardware adds on an
 // idle SM (several times that beside other FP64 work, which shares the SM's one FP64 unit), and
 // a restart of the scan above at every binade change, which a sum of mixed signs has every few
-// terms.  Here a block takes kBlockTile terms a step on the integer pipes, across binade changes:
-//   1. approximate prefix sums (fixed point, one scan) predict the binade of every running sum;
-//   2. with S_i in units of 2^-9 ulps of the frame's top binade, and g_i the ulp of S_i's
-//      predicted binade in that unit,
+// terms.  Here a block takes kScanTile terms a step on the integer pipes, across binade changes:
+//   1. the terms as integers in units of 2^-9 ulps of the frame's top binade (rounded down, a set
+//      last bit standing for the bits below) and one scan of them predict the binade of every
+//      running sum;
+//   2. with g_i the ulp of S_i's predicted binade in that unit,
 //          S_i = g_i · RNE((S_{i-1} + t_i) / g_i).
 //      Where g_i <= g_{i-1} and t_i is not halfway between multiples of g_i, that is S_{i-1} plus
 //      t_i rounded to g_i, whatever S_{i-1} is: a second scan adds these.  The others, "events"
 //      (ties, and steps into a higher binade, which round S_{i-1}'s own last bits), are few;
 //   3. one warp goes through the events in order (an integer add, a rounding and a subtraction
 //      each, about 50 clocks) and hands every position the correction of the last event before it;
-//   4. every position checks that its sum lies strictly inside its predicted binade: up to the
-//      first that does not, all are the sequential sum's bits, by induction.
+//   4. every position checks that its sum lies inside its predicted binade, not next to its ends:
+//      up to the first that does not, all are the sequential sum's bits, by induction.
 // The frame spans 8 binades (the starting sum's, four above, three below).  A step ends at the
-// first position outside it, after which a few terms take hardware adds.
-// Measured as the heavy kernel beside the edge phase: BA(2e6, 4) diffusion 217 µs -> 80 µs (the
-// warp scan on its 9 rows above 2048 terms against this one on all 264 from 400 up; the largest
-// has 6327), BA(1e5, 2) swing 47 µs for its 36 rows above 128 (the largest has 935; a thread
-// takes 56 to 75 µs for it, and the 256-term scan restarted at binade changes took 92 µs).
+// first position outside it (mostly a sum close to zero).
+// The heavy kernel alone, 36 rows of 129 to 935 terms of BA(1e5, 2) swing / 264 rows of 400 to 6327
+// terms of BA(2e6, 4) diffusion: 38 / 48 µs; with 256 threads of four terms, 64-bit binade tests
+// and a scan of their own for the predictions 71 / 52 µs.  A thread of the row phase takes 56 to
+// 75 µs for the 935-term row, and the 256-term warp scan took 164 µs for the 6327-term one.
+constexpr int kScanThreads = 128;
+constexpr int kScanWarps = kScanThreads / 32;
 constexpr int kBlockPer = 4;
-constexpr int kBlockTile = kBlock * kBlockPer;
+constexpr int kScanTile = kScanThreads * kBlockPer;
 // Position i of a tile in shared memory: one pad entry per thread's terms keeps the threads'
 // reads of their own terms free of bank conflicts.
 __device__ __forceinline__ int tile_at(int i) { return i + i / kBlockPer; }
-constexpr int kBlockTilePadded = kBlockTile + kBlockTile / kBlockPer;
+constexpr int kScanTilePadded = kScanTile + kScanTile / kBlockPer;
 constexpr int kFrameUp = 4, kFrameTop = 9, kFrameLow = 2;  // log2 of g: kFrameTop in the top binade
+// A step costs about as much as 48 hardware adds.  A step that advanced less is followed by a run
+// of them, doubled while that persists; a longer one by the two that bring a sum close to zero
+// back to the terms' size.
+constexpr int kScanShort = 48, kRunMin = 2, kRunShort = 32, kRunMax = 512;
 
 struct BlockScanShared {
-    int64_t approx[kWarpsPerBlock], total[kWarpsPerBlock];
-    int count[kWarpsPerBlock], emax[kWarpsPerBlock];
-    unsigned outside[kWarpsPerBlock], first_bad[kWarpsPerBlock];
+    int64_t term[kScanWarps], total[kScanWarps];
+    int count[kScanWarps];
+    unsigned outside[kScanWarps], first_bad[kScanWarps];
     int n_events;
     double sum;
     // events: the prefix before it (then the correction behind it), its term, log2 g
-    int64_t ev_prefix[kBlockTile], ev_term[kBlockTile];
-    int8_t ev_shift[kBlockTile];
+    int64_t ev_prefix[kScanTile], ev_term[kScanTile];
+    int8_t ev_shift[kScanTile];
 };
 
-__device__ __forceinline__ int64_t signed_of(uint64_t mag, uint64_t bits) {
-    return (bits & exact::kSign) ? -(int64_t)mag : (int64_t)mag;
+// The upper word of |m|, one too small for negative m whose lower word is not zero.
+__device__ __forceinline__ uint32_t abs_hi(int64_t m) {
+    const int32_t h = (int32_t)(m >> 32);
+    return (uint32_t)(h ^ (h >> 31));
 }
 
 // S + the n terms of `tile` (tile_at layout), in order; S is the same in every thread, and so
-// is the result.  All kBlock threads call it; `tile` is visible to all of them before.
+// is the result.  All kScanThreads threads call it; `tile` is visible to all of them before.
 static __device__ __forceinline__ double exact_scan_block(double S, const double* __restrict__ tile, int n,
                                                           BlockScanShared& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int base = tid * kBlockPer;
-    // this thread's terms: significands, exponent fields (subnormals: 1) and signs
-    uint64_t mag[kBlockPer], bits[kBlockPer];
+    // this thread's terms: signed significands and exponent fields (subnormals: 1)
+    int64_t sig[kBlockPer];
     int et[kBlockPer];
-    int emax = 0;
 #pragma unroll
     for (int i = 0; i < kBlockPer; ++i) {
-        bits[i] = base + i < n ? exact::to_bits(tile[tile_at(base + i)]) : 0;
-        const int e = (int)((bits[i] >> 52) & 0x7ff);
-        mag[i] = (bits[i] & exact::kFrac) | (e ? exact::kHidden : 0);
+        const uint64_t b = base + i < n ? exact::to_bits(tile[tile_at(base + i)]) : 0;
+        const int e = (int)((b >> 52) & 0x7ff);
+        const int64_t m = (int64_t)((b & exact::kFrac) | (e ? exact::kHidden : 0));
+        sig[i] = (b & exact::kSign) ? -m : m;
         et[i] = e ? e : 1;
-        emax = max(emax, e);
     }
-    emax = (int)__reduce_max_sync(kFull, (unsigned)emax);
-    if (lane == 0) sh.emax[warp] = emax;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < kWarpsPerBlock; ++w) emax = max(emax, sh.emax[w]);
-    int pos = 0, run_len = 8;
-    // > 0: the next run is this many hardware adds.  All of a tile with infinities or NaN; the
-    // first terms of a row, whose sum starts at zero.
-    int fallback = emax == 0x7ff ? n : ((exact::to_bits(S) << 1) == 0 ? run_len : 0);
+    int pos = 0, run_len = 0;
+    int fallback = (exact::to_bits(S) << 1) == 0 ? 8 : 0;  // > 0: the next run is this many hardware adds
     while (pos < n) {
         const uint64_t sb = exact::to_bits(S);
         const int eS = (int)((sb >> 52) & 0x7ff);
-        if (fallback == 0 && (eS < 16 || eS > 0x7ff - 32)) fallback = 1;  // zero, subnormal, near overflow, not finite
+        if (fallback == 0 && (eS < 16 || eS > 0x7ff - 32)) fallback = kRunShort;  // zero, subnormal, not finite
         if (fallback > 0) {  // one warp, so that the SM's FP64 unit serves this chain alone
             const int stop = min(n, pos + fallback);
             if (warp == 0) {
@@ -429,17 +430,27 @@ static __device__ __forceinline__ double exact_scan_block(double S, const double
             fallback = 0;
             continue;
         }
-        // 1. approximate prefix sums in units of 2^(EA - 1085): at most 1025 numbers below
-        //    2^(EA - 1034), so no sum overflows
-        const int EA = max(eS, emax) + 12;
-        const uint64_t magS = (sb & exact::kFrac) | exact::kHidden;
-        const int64_t aS = signed_of(magS >> min(63, EA - eS - 10), sb);
-        int64_t apx[kBlockPer];
+        // 1. the terms in frame units, and their scan
+        const int64_t mS = (int64_t)(((sb & exact::kFrac) | exact::kHidden) << (kFrameTop - kFrameUp));
+        const int64_t m0 = (sb & exact::kSign) ? -mS : mS;
+        int64_t term[kBlockPer];
         int64_t run = 0;
+        unsigned outside = 0xffffffffu;
 #pragma unroll
-        for (int i = 0; i < kBlockPer; ++i) {
-            if (base + i >= pos) run += signed_of(mag[i] >> min(63, EA - et[i] - 10), bits[i]);
-            apx[i] = run;
+        for (int i = kBlockPer - 1; i >= 0; --i) {
+            const int L = et[i] - eS + (kFrameTop - kFrameUp);  // significand · 2^L
+            int64_t t;
+            if (L >= 0) {
+                t = sig[i] << min(L, 10);
+            } else {
+                const int r = min(-L, 63);
+                t = sig[i] >> r;
+                t |= (int64_t)((t << r) != sig[i]);
+            }
+            const bool active = base + i >= pos;  // 0 behind the end of the tile
+            if (active && L > 10 && sig[i] != 0) outside = (unsigned)(base + i);
+            term[i] = active ? t : 0;
+            run += term[i];
         }
         int64_t x = run;
 #pragma unroll
@@ -447,45 +458,31 @@ static __device__ __forceinline__ double exact_scan_block(double S, const double
             const int64_t y = __shfl_up_sync(kFull, x, off);
             if (lane >= off) x += y;
         }
-        if (lane == 31) sh.approx[warp] = x;
+        if (lane == 31) sh.term[warp] = x;
         __syncthreads();
-        int64_t before = aS + (x - run);
-        for (int w = 0; w < warp; ++w) before += sh.approx[w];
-        // 2. predicted log2 g, rounded terms and events
-        auto log_g = [&](int64_t A) {  // of the binade of an approximate sum; 0: too small to tell
-            const uint64_t m = (uint64_t)(A < 0 ? -A : A);
-            if (m < (1ull << 22)) return 0;
-            const int e = EA - 62 + 63 - exact::clz64(m);
-            return max(0, min(kFrameTop + 1, e - eS + (kFrameTop - kFrameUp)));
-        };
-        int64_t term[kBlockPer], pre[kBlockPer];
+        int64_t before = m0 + (x - run);
+#pragma unroll
+        for (int w = 0; w < kScanWarps - 1; ++w)
+            if (w < warp) before += sh.term[w];
+        // 2. predicted log2 g (kFrameTop in the binade with |S| in [2^61, 2^62)), rounded terms, events
+        auto log_g = [](int64_t A) { return kFrameTop + 2 - exact::clz32(abs_hi(A)); };
+        int64_t pre[kBlockPer];
         int lg[kBlockPer];
-        unsigned events = 0, outside = 0xffffffffu;
-        int prev = max(kFrameLow, min(kFrameTop, log_g(before)));
+        unsigned events = 0;
+        int prev = log_g(before);
         run = 0;
 #pragma unroll
         for (int i = 0; i < kBlockPer; ++i) {
-            const int q = base + i;
-            lg[i] = log_g(before + apx[i]);
-            const int L = et[i] - eS + (kFrameTop - kFrameUp);  // t in frame units: significand · 2^L
-            const bool active = q >= pos && q < n;
-            if (active && (lg[i] < kFrameLow || lg[i] > kFrameTop || (L > 10 && mag[i] != 0))) outside = min(outside, (unsigned)q);
-            uint64_t m;
-            if (L >= 0) {
-                m = mag[i] << min(L, 10);
-            } else {  // the bits below the unit only count as "not zero" (the last bit set)
-                const int r = min(-L, 63);
-                m = mag[i] >> r;
-                m |= (uint64_t)((m << r) != mag[i]);
-            }
-            term[i] = active ? signed_of(m, bits[i]) : 0;
-            const int s = max(kFrameLow, min(kFrameTop, lg[i]));
-            const uint32_t g = 1u << s, low = (uint32_t)term[i] & (g - 1);
-            const bool event = active && (lg[i] > prev || low == g / 2);
+            before += term[i];
+            const int s = log_g(before);
+            if (base + i >= pos && base + i < n && (unsigned)(s - kFrameLow) > (unsigned)(kFrameTop - kFrameLow))
+                outside = min(outside, (unsigned)(base + i));
+            lg[i] = max(kFrameLow, min(kFrameTop, s));
+            const uint32_t g = 1u << lg[i], half = g >> 1;
+            const bool event = s > prev || ((uint32_t)term[i] & (g - 1)) == half;
             events |= (unsigned)event << i;
-            if (!event) run += (term[i] + (int64_t)(g / 2)) & ~(int64_t)(g - 1);
+            if (!event) run += (term[i] + (int64_t)half) & ~(int64_t)(g - 1);
             pre[i] = run;
-            lg[i] = s;
             prev = s;
         }
         x = run;
@@ -511,7 +508,7 @@ static __device__ __forceinline__ double exact_scan_block(double S, const double
         cnt -= mine;
         int P = n;
 #pragma unroll
-        for (int w = 0; w < kWarpsPerBlock; ++w) {
+        for (int w = 0; w < kScanWarps; ++w) {
             if (w < warp) {
                 before += sh.total[w];
                 cnt += sh.count[w];
@@ -533,14 +530,13 @@ static __device__ __forceinline__ double exact_scan_block(double S, const double
         if (P == 0 && tid == 0) sh.n_events = 0;
         __syncthreads();
         // 3. the events, in order
-        const int64_t m0 = signed_of(magS << (kFrameTop - kFrameUp), sb);
         if (warp == 0) {
             const int ne = sh.n_events;
             int64_t c = m0;
             int64_t b = sh.ev_prefix[0], t = sh.ev_term[0];
             int s = sh.ev_shift[0];
             for (int k = 0; k < ne; ++k) {
-                const int kn = min(k + 1, kBlockTile - 1);
+                const int kn = min(k + 1, kScanTile - 1);
                 const int64_t bn = sh.ev_prefix[kn], tn = sh.ev_term[kn];
                 const int sn = sh.ev_shift[kn];
                 const int64_t v = c + (b + t);
@@ -554,7 +550,9 @@ static __device__ __forceinline__ double exact_scan_block(double S, const double
             }
         }
         __syncthreads();
-        // 4. the sums, and the first position whose sum is not strictly inside its binade
+        // 4. the sums, and the first position whose sum is not inside its binade: the upper word
+        // of |S_i| has 22 or more bits of it, which must be those of the binade and neither all
+        // zero nor all one below the first
         int64_t val[kBlockPer];
         unsigned firstbad = 0xffffffffu;
 #pragma unroll
@@ -562,14 +560,17 @@ static __device__ __forceinline__ double exact_scan_block(double S, const double
             cnt += (int)((events >> i) & 1u);
             const bool in = base + i >= pos && base + i < P;
             val[i] = before + pre[i] + (cnt > 0 && in ? sh.ev_prefix[cnt - 1] : m0);
-            const uint64_t am = (uint64_t)(val[i] < 0 ? -val[i] : val[i]) >> lg[i];
-            if (in && (am < (1ull << 52) + 1 || am > (1ull << 53) - 2)) firstbad = min(firstbad, (unsigned)(base + i));
+            const uint32_t h = abs_hi(val[i]);
+            const int lz = exact::clz32(h);
+            const uint32_t low = (h << lz) & 0x7ffffe00u;
+            if (in && (kFrameTop + 2 - lz != lg[i] || low == 0 || low == 0x7ffffe00u))
+                firstbad = min(firstbad, (unsigned)(base + i));
         }
         firstbad = __reduce_min_sync(kFull, firstbad);
         if (lane == 0) sh.first_bad[warp] = firstbad;
         __syncthreads();
 #pragma unroll
-        for (int w = 0; w < kWarpsPerBlock; ++w) P = (int)min((unsigned)P, sh.first_bad[w]);
+        for (int w = 0; w < kScanWarps; ++w) P = (int)min((unsigned)P, sh.first_bad[w]);
         // positions [pos, P) are exact: the owner of P - 1 publishes the sum behind it
         if (P > pos) {
 #pragma unroll
@@ -583,10 +584,9 @@ static __device__ __forceinline__ double exact_scan_block(double S, const double
             __syncthreads();
             S = sh.sum;
         }
-        // behind a position outside the frame a run of hardware adds, longer while steps stay short
-        run_len = P - pos >= 64 ? 4 : min(64, 2 * run_len);
+        run_len = P - pos >= kScanShort ? 0 : min(kRunMax, max(kRunShort, 2 * run_len));
         pos = P;
-        if (pos < n) fallback = run_len;
+        if (pos < n) fallback = max(kRunMin, run_len);
         __syncthreads();  // sh is written again
     }
     return S;
