@@ -239,6 +239,8 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
     t.n_medium = (int32_t)medium.size();
     t.n_heavy = (int32_t)heavy.size();
     t.n_windows = (int32_t)win_ptr.size() - 1;
+    while (t.n_jvp_block < t.n_heavy + t.n_medium && deg[slot_vertex[t.n_jvp_block]] >= (uint32_t)kJvpBlockMin)
+        ++t.n_jvp_block;
     auto upload = [&](void** dptr, const void* hptr, size_t bytes) -> cudaError_t {
         cudaError_t err = cudaMalloc(dptr, std::max<size_t>(bytes, 16));
         if (err != cudaSuccess) return err;

@@ -89,6 +89,7 @@ constexpr int64_t heavy_min_deg(int64_t ninc) {
 constexpr int kWindow = 256;
 constexpr int kWarpRowMinF32 = 128;  // FP32 rows at least this long take a warp in the row phase
 constexpr int kLightRun = 128;
+constexpr int kJvpBlockMin = 256;  // rows at least this long take a block each in the JVP
 
 // Device-resident topology of one network.
 // Rows are stored in processing order ("slots"): heavy rows (by degree, descending), then
@@ -142,6 +143,7 @@ struct Topology {
     Incidence* incid = nullptr;      // [2ne] incidences in slot order, each row by edge id (fused path)
     int32_t* win_ptr = nullptr;      // [n_windows+1] first slot of each light window
     int32_t n_light = 0, n_medium = 0, n_heavy = 0, n_windows = 0;
+    int32_t n_jvp_block = 0;         // slots of at least kJvpBlockMin terms (the first ones)
     EdgeLayout edge;
 };
 
@@ -343,6 +345,11 @@ struct JacPlan {
     int32_t* colidx = nullptr;
     int32_t* long_slots = nullptr;  // slots of the rows that take a warp each
     int64_t n_long = 0;
+    // static edges and distinct columns in every row: the places of every term's neighbour column
+    // (-1: none) and of every slot's own column in the values
+    bool simple = false;
+    int32_t* term_place = nullptr;  // [2ne]
+    int32_t* own_place = nullptr;   // [nv]
     void* values = nullptr;         // Jacobian values kept for nd_jvp of batched handles
 };
 void free_jacobian(JacPlan* j);

@@ -18,10 +18,12 @@
 // voltage states of both endpoints of every incident line; the values come from dual
 // numbers carried through the component functions (jac_powergrid_kernel).
 //
-// Values: one thread per vertex row of up to 32 terms adds its terms' derivatives into its
-// row (found by binary search in the sorted columns), in the order of its terms; longer
-// rows take a warp each; one thread per ODE edge writes that edge's two rows.  For simple
-// graphs the result is deterministic.  Homogeneous handles
+// Values: where every row's columns are distinct (a simple graph, static edges), each term's
+// place in the values is found once, with the pattern, and one launch writes every entry
+// exactly once (jac_simple_kernel).  Otherwise one thread per vertex row of up to 32 terms adds
+// its terms' derivatives into its row (found by binary search in the sorted columns), in the
+// order of its terms; longer rows take a warp each; one thread per ODE edge writes that edge's
+// two rows.  For simple graphs the result is deterministic.  Homogeneous handles
 // get a batched view of their network (no scratch) built from their device topology.
 #include <algorithm>
 #include <string>
@@ -232,6 +234,145 @@ __global__ void __launch_bounds__(kJacBlock) jac_long_row_kernel(JacArgs<T> a, c
     if (lane == 0) jadd<T>(vals, cols, n, own, own_sum);
 }
 
+// ---- networks whose rows have distinct columns -------------------------------------------------
+// Vertex of a slot: its batch's kind, first state and parameter.
+struct JacVertex {
+    int kind, dim;
+    int64_t s, q;
+};
+template <typename T>
+__device__ __forceinline__ JacVertex jac_vertex(const JacArgs<T>& a, int64_t slot) {
+    const int64_t pos = __ldg(a.slot_vpos + slot);
+    const int b = find_batch(a.vb, pos);
+    JacVertex v;
+    v.kind = __ldg(a.vb.kind + b);
+    const int64_t r = pos - __ldg(a.vb.pos0 + b);
+    v.dim = v.kind == ND_V_SWING || v.kind == ND_V_SWING_UNIT ? 2 : 1;
+    v.s = __ldg(a.vb.s0 + b) + v.dim * r;
+    v.q = __ldg(a.vb.p0 + b) + (v.kind == ND_V_DIFFUSION ? 0 : (v.kind == ND_V_SWING ? 3 : 1)) * r;
+    return v;
+}
+
+// Place of column c in the row [r0, r0 + n) of the pattern; -1: not there.
+__device__ __forceinline__ int32_t jac_place(const int32_t* __restrict__ colidx, int32_t r0, int n, int32_t c) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(colidx + r0 + mid) < c) lo = mid + 1;
+        else hi = mid;
+    }
+    return n > 0 && __ldg(colidx + r0 + lo) == c ? r0 + lo : -1;
+}
+
+// The places of every term's neighbour column and of every row's own column, with the pattern.
+template <typename T>
+__global__ void __launch_bounds__(kJacBlock) jac_places_kernel(JacArgs<T> a, int32_t* __restrict__ term_place,
+                                                               int32_t* __restrict__ own_place) {
+    const int64_t w = ((int64_t)blockIdx.x * kJacBlock + threadIdx.x) >> 5;  // a warp per row
+    const int lane = threadIdx.x & 31;
+    if (w >= a.nv) return;
+    const JacVertex v = jac_vertex(a, w);
+    const int64_t row = v.s + v.dim - 1;
+    const int32_t r0 = __ldg(a.rowptr + row);
+    const int n = __ldg(a.rowptr + row + 1) - r0;
+    if (lane == 0) own_place[w] = jac_place(a.colidx, r0, n, (int32_t)v.s);
+    for (uint32_t j = __ldg(a.tptr + w) + lane; j < __ldg(a.tptr + w + 1); j += 32) {
+        const int32_t t = __ldg(a.tidx + j);
+        const int2 o = __ldg(a.eu + (t >> 1));
+        const bool none = !(t & 1) && __ldg(a.eb.coupling + find_batch(a.eb, t >> 1)) == ND_DIRECTED;
+        term_place[j] = none ? -1 : jac_place(a.colidx, r0, n, (t & 1) ? o.x : o.y);
+    }
+}
+
+// Every entry of the rows of static edges: a warp per row above kJacLongRow terms (n_long of them,
+// in `slots`, the first blocks), a thread per other row.  A term's neighbour entry is stored at
+// its place, the row's own entry is the sum of its terms' own derivatives in their order (lane
+// sums and a butterfly on the long rows), and the swing rows' two entries of ω are stored too:
+// no entry is cleared before or read.  On BA(1e5, 2) swing the values took 201 µs with the
+// binary searches, read-modify-writes and a launch per role, and 43 µs now; bound by the chain of
+// loads from a term to its neighbour's state.
+template <typename T>
+__global__ void __launch_bounds__(kJacBlock) jac_simple_kernel(JacArgs<T> a, const int32_t* __restrict__ slots,
+                                                               int64_t n_long, const int32_t* __restrict__ term_place,
+                                                               const int32_t* __restrict__ own_place) {
+    using A = Arith<T>;
+    constexpr int kWarps = kJacBlock / 32;
+    const int64_t long_blocks = (n_long + kWarps - 1) / kWarps;
+    const bool shared_row = (int64_t)blockIdx.x < long_blocks;
+    const int lane = threadIdx.x & 31;
+    int64_t slot;
+    if (shared_row) {
+        const int64_t w = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
+        if (w >= n_long) return;  // warp-uniform
+        slot = __ldg(slots + w);
+    } else {
+        slot = ((int64_t)blockIdx.x - long_blocks) * kJacBlock + threadIdx.x;
+        if (slot >= a.nv) return;
+    }
+    const uint32_t t0 = __ldg(a.tptr + slot), t1 = __ldg(a.tptr + slot + 1);
+    if (!shared_row && t1 - t0 > kJacLongRow) return;
+    const JacVertex v = jac_vertex(a, slot);
+    const bool first = !shared_row || lane == 0;
+    T scale = T(1);
+    if (v.dim == 2) {  // dθ = ω, and the row's own ω (see jac_vertex_kernel)
+        T dw = T(-1);
+        if (v.kind == ND_V_SWING) {
+            scale = A::div(T(1), __ldg(a.p + v.q));
+            dw = -A::mul(scale, __ldg(a.p + v.q + 1));
+        }
+        if (first) {
+            const int32_t r0 = __ldg(a.rowptr + v.s), r1 = __ldg(a.rowptr + v.s + 1);
+            a.values[r0] = T(1);  // the only column of dθ
+            // the ω column follows the own column, or is alone in a row without terms
+            const int32_t own = __ldg(own_place + slot);
+            a.values[own < 0 ? r1 : own + 1] = dw;
+        }
+    }
+    const T uv = __ldg(a.u + v.s);
+    constexpr int kB = 4;
+    const uint32_t step = shared_row ? 32 : 1;
+    T sum = T(0);
+    for (uint32_t j0 = t0 + (shared_row ? lane : 0); j0 < t1; j0 += kB * step) {
+        int32_t t[kB], place[kB];
+        T un[kB], w[kB];
+#pragma unroll
+        for (int i = 0; i < kB; ++i) {
+            const uint32_t j = j0 + i * step;
+            t[i] = j < t1 ? __ldg(a.tidx + j) : 0;
+            place[i] = j < t1 ? __ldg(term_place + j) : -1;
+        }
+#pragma unroll
+        for (int i = 0; i < kB; ++i) {
+            un[i] = w[i] = T(0);
+            if (place[i] < 0) continue;
+            const int64_t k = t[i] >> 1;
+            const int eb = find_batch(a.eb, k);
+            const int2 o = __ldg(a.eu + k);
+            un[i] = __ldg(a.u + ((t[i] & 1) ? o.x : o.y));
+            const int ek = __ldg(a.eb.kind + eb);
+            w[i] = ek == ND_E_DIFFUSION_UNIT ? T(1) : __ldg(a.p + __ldg(a.eb.p0 + eb) + (k - __ldg(a.eb.pos0 + eb)));
+            // ∂g/∂vs = -∂g/∂vd = c; cos is even, so the order of the difference does not matter
+            if (ek == ND_E_KURAMOTO) w[i] = A::times_cos(w[i], A::sub(un[i], uv));
+            // the destination's neighbour is the source: +c; the source's is the destination, with
+            // y_src = -y_dst again +c, and with y_src = y_dst (Symmetric) -c
+            if (!(t[i] & 1) && __ldg(a.eb.coupling + eb) == ND_SYMMETRIC) w[i] = -w[i];
+        }
+#pragma unroll
+        for (int i = 0; i < kB; ++i) {
+            if (place[i] < 0) continue;
+            const T d = A::mul(scale, w[i]);
+            a.values[place[i]] = d;
+            sum = A::sub(sum, d);
+        }
+    }
+    if (shared_row) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) sum = A::add(sum, __shfl_xor_sync(0xffffffffu, sum, off));
+    }
+    const int32_t own = __ldg(own_place + slot);
+    if (first && own >= 0) a.values[own] = sum;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kJacBlock) jac_ode_edge_kernel(JacArgs<T> a) {
     using A = Arith<T>;
@@ -397,6 +538,27 @@ int build_view(nd_handle* h, BatchedNet* view) {
     return build_batched(&d, 0, view);
 }
 
+template <typename T>
+JacArgs<T> jac_args(const nd_handle* h, void* values, const void* u, const void* p) {
+    const JacPlan& J = h->jac;
+    const BatchedNet& b = h->batched.enabled ? h->batched : J.view;
+    JacArgs<T> a;
+    a.values = static_cast<T*>(values);
+    a.u = static_cast<const T*>(u);
+    a.p = static_cast<const T*>(p);
+    a.rowptr = J.rowptr;
+    a.colidx = J.colidx;
+    a.nv = b.nv;
+    a.ne = b.ne;
+    a.vb = b.dvb;
+    a.eb = b.deb;
+    a.eu = b.eu;
+    a.tptr = b.tptr;
+    a.tidx = b.tidx;
+    a.slot_vpos = b.slot_vpos;
+    return a;
+}
+
 // Pattern of the Jacobian (see the file comment), built on the host from the batched
 // structure.
 int build_plan(nd_handle* h) {
@@ -473,12 +635,18 @@ int build_plan(nd_handle* h) {
             rows[es + i].push_back((int32_t)(es + i));
         }
     }
+    // every row's columns distinct: each term brings one column besides the row's own
+    J.simple = b.depth == 1;
+    for (int32_t k : b.eb.kind) J.simple = J.simple && !is_ode(k);
     J.rowptr_h.assign(dim + 1, 0);
     int64_t nnz = 0;
     for (int64_t i = 0; i < dim; ++i) {
         std::vector<int32_t>& r = rows[i];
+        const size_t pushed = r.size();  // of a vertex's aggregated row: twice its terms, + 1 (swing ω)
         std::sort(r.begin(), r.end());
         r.erase(std::unique(r.begin(), r.end()), r.end());
+        const size_t terms = pushed / 2;
+        J.simple = J.simple && r.size() == (terms ? terms + 1 : 0) + (pushed & 1);
         nnz += (int64_t)r.size();
         if (nnz > (int64_t)INT32_MAX) return fail(ND_ERR_UNSUPPORTED, "nd_jacobian: more than 2^31-1 nonzeros");
         J.rowptr_h[i + 1] = (int32_t)nnz;
@@ -500,6 +668,15 @@ int build_plan(nd_handle* h) {
         (J.n_long > 0 && (err = cudaMemcpy(J.long_slots, long_slots.data(), J.n_long * sizeof(int32_t),
                                            cudaMemcpyHostToDevice)) != cudaSuccess))
         return cuda_fail(err, "nd_jacobian: pattern upload");
+    if (J.simple) {
+        if ((err = cudaMalloc(&J.term_place, std::max<int64_t>(2 * ne, 1) * sizeof(int32_t))) != cudaSuccess ||
+            (err = cudaMalloc(&J.own_place, nv * sizeof(int32_t))) != cudaSuccess)
+            return cuda_fail(err, "nd_jacobian: pattern upload");
+        jac_places_kernel<double><<<(unsigned)((nv * 32 + kJacBlock - 1) / kJacBlock), kJacBlock>>>(
+            jac_args<double>(h, nullptr, nullptr, nullptr), J.term_place, J.own_place);
+        if ((err = cudaGetLastError()) != cudaSuccess || (err = cudaStreamSynchronize(nullptr)) != cudaSuccess)
+            return cuda_fail(err, "nd_jacobian: places of the terms");
+    }
     J.ready = true;
     return ND_OK;
 }
@@ -508,20 +685,12 @@ template <typename T>
 cudaError_t launch_values(nd_handle* h, void* values, const void* u, const void* p, cudaStream_t s) {
     const JacPlan& J = h->jac;
     const BatchedNet& b = h->batched.enabled ? h->batched : J.view;
-    JacArgs<T> a;
-    a.values = static_cast<T*>(values);
-    a.u = static_cast<const T*>(u);
-    a.p = static_cast<const T*>(p);
-    a.rowptr = J.rowptr;
-    a.colidx = J.colidx;
-    a.nv = b.nv;
-    a.ne = b.ne;
-    a.vb = b.dvb;
-    a.eb = b.deb;
-    a.eu = b.eu;
-    a.tptr = b.tptr;
-    a.tidx = b.tidx;
-    a.slot_vpos = b.slot_vpos;
+    const JacArgs<T> a = jac_args<T>(h, values, u, p);
+    if (J.simple) {
+        const int64_t blocks = (J.n_long * 32 + kJacBlock - 1) / kJacBlock + (b.nv + kJacBlock - 1) / kJacBlock;
+        jac_simple_kernel<T><<<(unsigned)blocks, kJacBlock, 0, s>>>(a, J.long_slots, J.n_long, J.term_place, J.own_place);
+        return cudaGetLastError();
+    }
     cudaError_t err = cudaMemsetAsync(values, 0, std::max<int64_t>(J.nnz, 1) * sizeof(T), s);
     if (err != cudaSuccess) return err;
     if (b.depth == 2) {
@@ -532,7 +701,9 @@ cudaError_t launch_values(nd_handle* h, void* values, const void* u, const void*
     if (J.n_long > 0)
         jac_long_row_kernel<T><<<(unsigned)((J.n_long * 32 + kJacBlock - 1) / kJacBlock), kJacBlock, 0, s>>>(
             a, J.long_slots, J.n_long);
-    if (b.ne > 0) jac_ode_edge_kernel<T><<<(unsigned)((b.ne + kJacBlock - 1) / kJacBlock), kJacBlock, 0, s>>>(a);
+    bool ode = false;
+    for (int32_t k : b.eb.kind) ode = ode || is_ode(k);
+    if (ode) jac_ode_edge_kernel<T><<<(unsigned)((b.ne + kJacBlock - 1) / kJacBlock), kJacBlock, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -586,6 +757,8 @@ void free_jacobian(JacPlan* j) {
     cudaFree(j->rowptr);
     cudaFree(j->colidx);
     cudaFree(j->long_slots);
+    cudaFree(j->term_place);
+    cudaFree(j->own_place);
     cudaFree(j->values);
     *j = JacPlan{};
 }

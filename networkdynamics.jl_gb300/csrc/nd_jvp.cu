@@ -9,10 +9,13 @@
 // and AntiSymmetric hands -d(y_dst) to the source, so at row v with neighbour n every
 // incidence contributes c (v_n - v_v) with c = w, 1 or K cos(θ_n - θ_v).  Vertices:
 //   diffusion / kuramoto   jv = Σ                  swing   jv_θ = v_ω,  jv_ω = (Σ - D v_ω) / M
-// One thread per row over the slot-ordered CSR, rows summed in edge order; rows of degree
-// above 32 (the first slots) take a warp each.
-#include <algorithm>
-
+// One launch over the slot-ordered CSR (rows by degree, the longest first): a block per row of
+// kJvpBlockMin terms and more, a warp per row above 32, a thread per row for the rest, which
+// sums in edge order.  A row is bound by the latency of its gathers (the neighbour, then its
+// state, direction and line weight), so each thread asks for four terms at a time, and the
+// longest rows start first and are split widest: as two launches with a warp for the longest
+// row, BA(5e5, 2) swing took 126 + 50 µs, now 53; a block from 256 terms on (8 round trips for a
+// warp, one or two for the block).
 #include "nd_components.cuh"
 #include "nd_internal.h"
 
@@ -21,21 +24,6 @@ namespace nd {
 int jacobian_times(nd_handle* h, void* jv, const void* u, const void* p, const void* v, cudaStream_t s);
 
 namespace {
-
-// Contribution c (v_n - v_v) of one incidence (neighbour n) to row v.
-template <typename T, int VK, int EK>
-__device__ __forceinline__ T jvp_term(int2 inc, T uv, T dv, const T* __restrict__ u, const T* __restrict__ pe,
-                                      const T* __restrict__ vv) {
-    using A = Arith<T>;
-    constexpr int DV = VertexDims<VK>::dim;
-    const int64_t n = inc.x;
-    const int32_t e = inc.y & 0x7fffffff;
-    T c;
-    if constexpr (EK == ND_E_DIFFUSION) c = pe[e];
-    else if constexpr (EK == ND_E_DIFFUSION_UNIT) c = T(1);
-    else c = A::times_cos(pe[e], A::sub(u[n * DV], uv));
-    return A::mul(c, A::sub(vv[n * DV], dv));
-}
 
 template <typename T, int VK>
 __device__ __forceinline__ void jvp_vertex(int64_t v, T acc, const T* __restrict__ pv, const T* __restrict__ vv,
@@ -50,66 +38,91 @@ __device__ __forceinline__ void jvp_vertex(int64_t v, T acc, const T* __restrict
     }
 }
 
-// Rows [first, nv) of the slot order, a thread each.
+constexpr int kJvpBlock = 256;
+
+// Σ over the terms k, k + step, ... < end of a row, four in flight.
 template <typename T, int VK, int EK>
-__global__ void jvp_kernel(int64_t first, int64_t nv, const uint32_t* __restrict__ slot_ptr,
-                           const int32_t* __restrict__ slot_vertex, const int2* __restrict__ incid,
-                           const T* __restrict__ u, const T* __restrict__ p, const T* __restrict__ vv,
-                           T* __restrict__ jv) {
+__device__ __forceinline__ T jvp_sum(uint32_t k, uint32_t end, uint32_t step, const int2* __restrict__ incid, T uv, T dv,
+                                     const T* __restrict__ u, const T* __restrict__ pe, const T* __restrict__ vv) {
     using A = Arith<T>;
     constexpr int DV = VertexDims<VK>::dim;
-    const T* pe = p + nv * VertexDims<VK>::pdim;
-    for (int64_t s = first + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < nv;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t v = slot_vertex[s];
-        const T uv = u[v * DV], dv = vv[v * DV];
-        T acc = T(0);
-        for (uint32_t k = slot_ptr[s]; k < slot_ptr[s + 1]; ++k)
-            acc = A::add(acc, jvp_term<T, VK, EK>(incid[k], uv, dv, u, pe, vv));
-        jvp_vertex<T, VK>(v, acc, p, vv, jv);
+    constexpr int kB = 4;
+    T acc = T(0);
+    for (; k < end; k += kB * step) {
+        int2 inc[kB];
+        T un[kB], dn[kB], w[kB];
+#pragma unroll
+        for (int j = 0; j < kB; ++j) inc[j] = k + j * step < end ? __ldg(incid + k + j * step) : int2{-1, 0};
+#pragma unroll
+        for (int j = 0; j < kB; ++j) {
+            un[j] = dn[j] = w[j] = T(0);
+            if (inc[j].x < 0) continue;
+            const int64_t n = (int64_t)inc[j].x * DV;
+            un[j] = EK == ND_E_KURAMOTO ? __ldg(u + n) : T(0);
+            dn[j] = __ldg(vv + n);
+            w[j] = EK == ND_E_DIFFUSION_UNIT ? T(1) : __ldg(pe + (inc[j].y & 0x7fffffff));
+        }
+#pragma unroll
+        for (int j = 0; j < kB; ++j) {
+            if (inc[j].x < 0) continue;
+            const T c = EK == ND_E_KURAMOTO ? A::times_cos(w[j], A::sub(un[j], uv)) : w[j];
+            acc = A::add(acc, EK == ND_E_DIFFUSION_UNIT ? A::sub(dn[j], dv) : A::mul(c, A::sub(dn[j], dv)));
+        }
     }
+    return acc;
 }
 
-// Rows [0, n_long) of the slot order (degree above 32: medium and heavy rows), a warp
-// each: lane partial sums and a butterfly.
 template <typename T, int VK, int EK>
-__global__ void jvp_warp_kernel(int64_t n_long, int64_t nv, const uint32_t* __restrict__ slot_ptr,
-                                const int32_t* __restrict__ slot_vertex, const int2* __restrict__ incid,
-                                const T* __restrict__ u, const T* __restrict__ p, const T* __restrict__ vv,
-                                T* __restrict__ jv) {
+__global__ void __launch_bounds__(kJvpBlock) jvp_kernel(int64_t n_block, int64_t n_long, int64_t nv,
+                                                        const uint32_t* __restrict__ slot_ptr,
+                                                        const int32_t* __restrict__ slot_vertex,
+                                                        const int2* __restrict__ incid, const T* __restrict__ u,
+                                                        const T* __restrict__ p, const T* __restrict__ vv,
+                                                        T* __restrict__ jv) {
     using A = Arith<T>;
     constexpr int DV = VertexDims<VK>::dim;
+    constexpr int kWarps = kJvpBlock / 32;
     const T* pe = p + nv * VertexDims<VK>::pdim;
-    const int lane = threadIdx.x & 31;
-    const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (s >= n_long) return;  // warp-uniform
-    const int64_t v = slot_vertex[s];
-    const T uv = u[v * DV], dv = vv[v * DV];
-    T acc = T(0);
-    for (uint32_t k = slot_ptr[s] + lane; k < slot_ptr[s + 1]; k += 32)
-        acc = A::add(acc, jvp_term<T, VK, EK>(incid[k], uv, dv, u, pe, vv));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t b = blockIdx.x, warp_blocks = (n_long - n_block + kWarps - 1) / kWarps;
+    // how many lanes share a row: the block, a warp, or one
+    const int share = b < n_block ? kJvpBlock : (b < n_block + warp_blocks ? 32 : 1);
+    const int64_t s = share == kJvpBlock ? b
+                      : share == 32      ? n_block + (b - n_block) * kWarps + warp
+                                         : n_long + (b - n_block - warp_blocks) * kJvpBlock + tid;
+    if (s >= (share == 32 ? n_long : nv)) return;  // never for a block's row: warp-uniform where a warp shares
+    const int64_t v = __ldg(slot_vertex + s);
+    const T uv = __ldg(u + v * DV), dv = __ldg(vv + v * DV);
+    const int first = share == kJvpBlock ? tid : (share == 32 ? lane : 0);
+    T acc = jvp_sum<T, VK, EK>(__ldg(slot_ptr + s) + first, __ldg(slot_ptr + s + 1), share, incid, uv, dv, u, pe, vv);
+    if (share > 1) {
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc = A::add(acc, __shfl_xor_sync(0xffffffffu, acc, off));
-    if (lane == 0) jvp_vertex<T, VK>(v, acc, p, vv, jv);
+        for (int off = 16; off > 0; off >>= 1) acc = A::add(acc, __shfl_xor_sync(0xffffffffu, acc, off));
+        if (share == kJvpBlock) {
+            __shared__ T red[kWarps];
+            if (lane == 0) red[warp] = acc;
+            __syncthreads();
+            acc = red[0];
+#pragma unroll
+            for (int w = 1; w < kWarps; ++w) acc = A::add(acc, red[w]);
+        }
+    }
+    if (first == 0) jvp_vertex<T, VK>(v, acc, p, vv, jv);
 }
 
 template <typename T>
 cudaError_t launch_jvp(const nd_handle* h, const void* u, const void* p, const void* v, void* jv, cudaStream_t s) {
     const Topology& t = h->topo;
     const int64_t n_long = (int64_t)t.n_heavy + t.n_medium;  // the first slots: degree > 32
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((t.nv - n_long + 255) / 256, 152 * 16));
-    const unsigned wgrid = (unsigned)((n_long * 32 + 255) / 256);
+    const int64_t n_block = t.n_jvp_block, warps = kJvpBlock / 32;
+    const unsigned grid = (unsigned)(n_block + (n_long - n_block + warps - 1) / warps +
+                                     (t.nv - n_long + kJvpBlock - 1) / kJvpBlock);
     const int2* inc = reinterpret_cast<const int2*>(t.incid);
 #define ND_CASE(VK, EK)                                                                                          \
     if (h->vertex_kind == VK && h->edge_kind == EK) {                                                             \
-        if (n_long > 0)                                                                                           \
-            jvp_warp_kernel<T, VK, EK><<<wgrid, 256, 0, s>>>(n_long, t.nv, t.slot_ptr, t.slot_vertex, inc,        \
-                                                            static_cast<const T*>(u), static_cast<const T*>(p),   \
-                                                            static_cast<const T*>(v), static_cast<T*>(jv));       \
-        if (t.nv > n_long)                                                                                        \
-            jvp_kernel<T, VK, EK><<<grid, 256, 0, s>>>(n_long, t.nv, t.slot_ptr, t.slot_vertex, inc,              \
-                                                      static_cast<const T*>(u), static_cast<const T*>(p),         \
-                                                      static_cast<const T*>(v), static_cast<T*>(jv));             \
+        jvp_kernel<T, VK, EK><<<grid, kJvpBlock, 0, s>>>(n_block, n_long, t.nv, t.slot_ptr, t.slot_vertex, inc,   \
+                                                         static_cast<const T*>(u), static_cast<const T*>(p),      \
+                                                         static_cast<const T*>(v), static_cast<T*>(jv));          \
         return cudaGetLastError();                                                                                \
     }
     ND_CASE(ND_V_DIFFUSION, ND_E_DIFFUSION)
