@@ -9,6 +9,7 @@ ext/NetworkDynamicsCUDAExt.jl:16-45) creates the device handle in libnd_b200.so.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import operator
 from typing import Sequence, Union
@@ -72,6 +73,15 @@ class GB300Execution(ExecutionStyle):
         return f"GB300Execution({', '.join(opts)})"
 
 
+def _raw_stream(stream) -> int:
+    """The cudaStream_t of `stream`, or of torch's current stream (without building a
+    torch.cuda.Stream object for it on every call)."""
+    if stream is not None:
+        return stream.cuda_stream
+    import torch
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
 def iscudacompatible(x) -> bool:
     return isinstance(x, (GB300Execution, GB300Aggregator))
 
@@ -96,11 +106,17 @@ def get_aggr_constructor(agg: GB300Aggregator) -> GB300Aggregator:
     return GB300Aggregator(agg.f)
 
 
-_TORCH_DT = None
+_torch_codes = {}  # torch dtype -> code, filled on first use (torch is imported late)
 
 
 def _dtype_code(dtype) -> int:
     import torch
+    if type(dtype) is torch.dtype:
+        if not _torch_codes:
+            _torch_codes.update({torch.float64: capi.ND_F64, torch.float32: capi.ND_F32})
+        code = _torch_codes.get(dtype)
+        if code is not None:
+            return code
     if dtype in (torch.float64, np.float64, "float64", "f64"):
         return capi.ND_F64
     if dtype in (torch.float32, np.float32, "float32", "f32"):
@@ -218,6 +234,7 @@ class Network:
         self._layout()
         self._handle = None
         self._dtype = None
+        self._jac_index = None  # (crow, col) of the Jacobian on the device, see jacobian()
         if dtype is not None:
             self._create(dtype)
 
@@ -386,29 +403,27 @@ class Network:
             if not (isinstance(x, torch.Tensor) and x.is_cuda and x.is_contiguous()):
                 raise capi.ArgumentError(capi.ND_ERR_ARG, f"{name} must be a contiguous CUDA tensor")
         code = _dtype_code(u.dtype)
-        if _dtype_code(du.dtype) != code:
+        if du.dtype is not u.dtype and _dtype_code(du.dtype) != code:
             raise capi.ArgumentError(capi.ND_ERR_DTYPE, "du and u have different element types")
         if p is None or (hasattr(p, "numel") and p.numel() == 0):
             p_ptr, n_p = None, 0
         else:
             if not (isinstance(p, torch.Tensor) and p.is_cuda and p.is_contiguous()):
                 raise capi.ArgumentError(capi.ND_ERR_ARG, "p must be a contiguous CUDA tensor")
-            if _dtype_code(p.dtype) != code:
+            if p.dtype is not u.dtype and _dtype_code(p.dtype) != code:
                 raise capi.ArgumentError(capi.ND_ERR_DTYPE, "p has a different element type than u")
             p_ptr, n_p = p.data_ptr(), p.numel()
-        s = stream if stream is not None else torch.cuda.current_stream()
-        capi.check(self._lib.nd_rhs(self.handle, code, du.data_ptr(), du.numel(), u.data_ptr(), u.numel(),
-                                    p_ptr, n_p, float(t), C.c_void_p(s.cuda_stream)))
+        rc = self._lib.nd_rhs(self.handle, code, du.data_ptr(), du.numel(), u.data_ptr(), u.numel(), p_ptr, n_p,
+                              float(t), _raw_stream(stream))
+        if rc != capi.ND_OK:
+            capi.check(rc)
         return None
 
 
 def jvp(nw: Network, jv, u, p, v, t=0.0, stream=None):
     """jv = (∂f/∂u)(u, p, t) · v with the analytic library derivatives (CUDA tensors)."""
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
     capi.check(nw._lib.nd_jvp(nw.handle, _dtype_code(u.dtype), jv.data_ptr(), u.data_ptr(),
-                              p.data_ptr() if p is not None else None, v.data_ptr(), float(t),
-                              C.c_void_p(s.cuda_stream)))
+                              p.data_ptr() if p is not None else None, v.data_ptr(), float(t), _raw_stream(stream)))
 
 
 def jacobian_pattern(nw: Network):
@@ -428,15 +443,20 @@ def jacobian(nw: Network, u, p, t=0.0, stream=None):
     """∂f/∂u at (u, p, t) with the analytic derivatives of the library components, as a
     torch sparse CSR tensor on u's device (values in the network's precision)."""
     import torch
-    rowptr, colidx = jacobian_pattern(nw)
-    values = torch.empty(len(colidx), dtype=u.dtype, device=u.device)
-    s = stream if stream is not None else torch.cuda.current_stream()
+    # the pattern is the network's: its index tensors go to the device once, and every call
+    # hands out copies of its own
+    index = nw._jac_index
+    if index is None or index[0].device != u.device:
+        rowptr, colidx = jacobian_pattern(nw)
+        index = nw._jac_index = tuple(torch.from_numpy(x.astype(np.int64)).to(u.device) for x in (rowptr, colidx))
+    # every tensor of the result belongs to the stream that fills it
+    with contextlib.nullcontext() if stream is None else torch.cuda.stream(stream):
+        crow, col = (x.clone() for x in index)
+        values = torch.empty(col.numel(), dtype=u.dtype, device=u.device)
     pp = p.data_ptr() if p is not None and p.numel() else None
     capi.check(nw._lib.nd_jacobian(nw.handle, _dtype_code(u.dtype), values.data_ptr(), u.data_ptr(), pp, float(t),
-                                   C.c_void_p(s.cuda_stream)))
-    return torch.sparse_csr_tensor(torch.from_numpy(rowptr.astype(np.int64)).to(u.device),
-                                   torch.from_numpy(colidx.astype(np.int64)).to(u.device), values,
-                                   size=(nw.dim, nw.dim))
+                                   _raw_stream(stream)))
+    return torch.sparse_csr_tensor(crow, col, values, size=(nw.dim, nw.dim))
 
 
 def adapt(nw: Network, dtype) -> Network:
@@ -449,6 +469,7 @@ def adapt(nw: Network, dtype) -> Network:
     out.__dict__.update({k: v for k, v in nw.__dict__.items() if k not in ("_handle", "_dtype", "_lib")})
     out._handle = None
     out._dtype = None
+    out._jac_index = None
     out._create(dtype)
     ex = nw.execution
     if ex.sum_order != "sequential":
