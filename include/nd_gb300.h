@@ -209,9 +209,9 @@ int nd_set_sum_order(nd_handle* h, int order);
 
 /* Kernel layout of the RHS.  ND_LAYOUT_AUTO (default) evaluates each edge once in edge
  * order and then sums the rows (two phases; needs the canonical edge list of an
- * undirected Graphs.jl graph: sorted by source, src < dst); other edge lists, or
- * ND_LAYOUT_FUSED, use one fused kernel over the destination-sorted CSR.  Both give the
- * same bits. */
+ * undirected Graphs.jl graph: sorted by source, src < dst); small networks (up to 1.05e6
+ * edges in FP64, 2.1e6 in FP32), other edge lists, or ND_LAYOUT_FUSED, use one fused kernel over
+ * the destination-sorted CSR.  Both give the same bits in FP64. */
 enum nd_layout { ND_LAYOUT_AUTO = 0, ND_LAYOUT_FUSED = 1 };
 int nd_set_layout(nd_handle* h, int layout);
 

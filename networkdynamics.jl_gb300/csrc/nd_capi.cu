@@ -165,16 +165,24 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
     // light rows in runs of consecutive vertices, are cut into windows of at most kWindow
     // rows and kWindowIncidences incidences and sorted by degree (descending, stable)
     // inside each window.
+    bool small = edge_elem > 0 && 2 * ne <= fused_max_incidences(edge_elem);
+    if (small && edge_elem == 8) {
+        int64_t dense = 0;
+        for (int64_t v = 0; v < nv; ++v)
+            if (deg[v] > (uint32_t)kFusedDenseRow) dense += deg[v];
+        small = dense <= ne;
+    }
     const bool canonical = edge_elem > 0 && ne > 0 && is_canonical(ne, src, dst);
+    const int64_t win_inc = small ? fused_window_incidences(2 * ne) : kWindowIncidences;
     int64_t heavy_min = kMediumMaxDeg + 1;
-    if (edge_elem == 8 && canonical) {
+    if (small || (edge_elem == 8 && canonical)) {
         // not where rows that long are the bulk of the network (a dense graph: its rows have a
         // kernel of their own)
-        const int64_t h = heavy_min_deg(2 * ne);
+        const int64_t h = small ? (edge_elem == 8 ? kFusedMaxRow : kFusedMaxRowF32) + 1 : heavy_min_deg(2 * ne);
         int64_t inc = 0;
         for (int64_t v = 0; v < nv; ++v)
             if (deg[v] >= (uint32_t)h) inc += deg[v];
-        if (8 * inc <= 2 * ne) heavy_min = h;
+        if (8 * inc <= 2 * ne || (small && edge_elem == 4)) heavy_min = h;
     }
     std::vector<int32_t> light, medium, heavy;
     light.reserve(nv);
@@ -203,7 +211,7 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
         for (size_t i = 0; i < windowed.size(); ++i) {
             const uint32_t d = deg[windowed[i]];
             // windows never mix medium and light rows
-            if (i - w0 == (size_t)kWindow || inc + d > (uint32_t)kWindowIncidences || (i == medium.size() && i > w0)) {
+            if (i - w0 == (size_t)kWindow || (inc + d > (uint32_t)win_inc && i > w0) || (i == medium.size() && i > w0)) {
                 std::stable_sort(windowed.begin() + w0, windowed.begin() + i, by_degree);
                 win_ptr.push_back((int32_t)i);
                 w0 = i;
@@ -239,6 +247,7 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
     t.n_medium = (int32_t)medium.size();
     t.n_heavy = (int32_t)heavy.size();
     t.n_windows = (int32_t)win_ptr.size() - 1;
+    t.small = small;
     while (t.n_jvp_block < t.n_heavy + t.n_medium && deg[slot_vertex[t.n_jvp_block]] >= (uint32_t)kJvpBlockMin)
         ++t.n_jvp_block;
     auto upload = [&](void** dptr, const void* hptr, size_t bytes) -> cudaError_t {
@@ -256,7 +265,7 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
         free_topology(&t);
         return cuda_fail(err, "upload of the network topology");
     }
-    if (canonical) {
+    if (canonical && !small) {
         EdgeLayoutHost h;
         build_edge_layout(nv, ne, src, dst, h);
         // the row records and the padded loc array, in slot order of the rows
@@ -613,7 +622,9 @@ int nd_rhs(nd_handle* h, int dtype, void* du, int64_t n_du, const void* u, int64
     a.dense_rows = el.dense_rows ? 1 : 0;
     a.n_warp_f32 = el.n_warp_f32;
     const bool edge = el.enabled && h->edge_path;
-    const bool split = h->topo.n_heavy > 0;  // heavy rows: their own kernel, on the side stream
+    // heavy rows: their own kernel, on the side stream; in FP32 on small networks the first blocks
+    // of the fused launch
+    const bool split = h->topo.n_heavy > 0 && !(h->topo.small && h->dtype == ND_F32);
     a.heavy_separate = split ? 1 : 0;
     const int64_t main_rows = (split ? 0 : h->topo.n_heavy) + h->topo.n_windows;
     cudaError_t err = cudaSuccess;

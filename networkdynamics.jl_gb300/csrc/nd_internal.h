@@ -86,6 +86,28 @@ constexpr int64_t heavy_min_deg(int64_t ninc) {
     const int64_t d = ninc / 40000;
     return 1 + (d < 128 ? 128 : (d > kMediumMaxDeg ? kMediumMaxDeg : d));
 }
+// Networks of up to this many incidences take the fused kernel whatever their edge list: their
+// data stay in L2, so evaluating an edge once per end costs less than a second launch and the
+// trip of its value through memory.  Fused / two-phase, µs per RHS call:
+//   FP64  Kuramoto WS(1e3, 10) 5.8 / 16.5, WS(2e5, 10) 28.8 / 28.8, swing BA(1e4, 2) 20.6 / 24.4,
+//         diffusion BA(2e5, 4) 44.5 / 46.1, BA(5e5, 4) 58.3 / 53.5
+//   FP32  Kuramoto WS(1e3, 10) 5.9 / 12.4, swing BA(1e5, 2) 14.4 / 20.6, diffusion BA(5e5, 4) 34.4 / 35.7
+// Not in FP64 where rows above kFusedDenseRow terms hold most incidences (a dense graph, whose
+// rows have a prefetching kernel in the two-phase layout): WS(1000, 500) 28.7 / 34.9, WS(1900, 950)
+// 75.9 / 55.4.
+constexpr int64_t fused_max_incidences(int elem) { return elem == 8 ? 2100000 : 4200000; }
+constexpr int kFusedDenseRow = 512;
+// Their windows shrink so that there are about two per SM, and their long rows stay in the
+// windows up to kFusedMaxRow terms: a thread adds them from shared memory at 36 ns a term in FP64
+// (10 µs for 256), less than the launch on the side stream and the block scan of a row that
+// short (diffusion BA(1e4, 4), rows up to 488 terms: 24.7 µs with all in windows, 16.5 with those
+// above 256 in the heavy kernel).  Longer rows: FP64 as above, FP32 a block each in the same
+// launch, from 129 terms on.
+constexpr int kFusedMaxRow = 256, kFusedMaxRowF32 = 128;
+constexpr int64_t fused_window_incidences(int64_t ninc) {
+    const int64_t w = ninc / 304;
+    return w < 256 ? 256 : (w > 2048 ? 2048 : w);
+}
 constexpr int kWindow = 256;
 constexpr int kWarpRowMinF32 = 128;  // FP32 rows at least this long take a warp in the row phase
 constexpr int kLightRun = 128;
@@ -144,6 +166,7 @@ struct Topology {
     int32_t* win_ptr = nullptr;      // [n_windows+1] first slot of each light window
     int32_t n_light = 0, n_medium = 0, n_heavy = 0, n_windows = 0;
     int32_t n_jvp_block = 0;         // slots of at least kJvpBlockMin terms (the first ones)
+    bool small = false;              // fused kernel whatever the edge list (fused_max_incidences)
     EdgeLayout edge;
 };
 

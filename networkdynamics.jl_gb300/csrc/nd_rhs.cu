@@ -147,7 +147,13 @@ __device__ __forceinline__ void window_block(const RhsArgs& a, int win, unsigned
         beg = (int)(__ldg(a.slot_ptr + s) - i0);
         end = (int)(__ldg(a.slot_ptr + s + 1) - i0);
         s_uv[tid] = ld_hint(u + v * DV, keep);
-        for (int j = beg; j < end; ++j) s_owner[j] = (uint8_t)tid;
+        if (end - beg <= kLightMaxDeg)
+            for (int j = beg; j < end; ++j) s_owner[j] = (uint8_t)tid;
+    }
+    // a long row's incidences are marked by its warp
+    for (unsigned m = __ballot_sync(kFull, end - beg > kLightMaxDeg); m; m &= m - 1) {
+        const int l = __ffs(m) - 1, e = __shfl_sync(kFull, end, l);
+        for (int j = __shfl_sync(kFull, beg, l) + (tid & 31); j < e; j += 32) s_owner[j] = (uint8_t)((tid & ~31) + l);
     }
     __syncthreads();
     // phase A: the edge terms, one incidence per thread: coalesced incidence loads, many

@@ -38,8 +38,8 @@ class GB300Execution(ExecutionStyle):
     - ``sum_order``: "sequential" (default; the bits of SequentialAggregator, with the exact
       scan at hubs), "sequential_hw" (the same bits with hardware adds at hubs) or "tree"
       (a deterministic warp tree at hubs; not bitwise);
-    - ``layout``: "auto" (two-phase edge-centric kernels for canonical edge lists, else the
-      fused kernel) or "fused";
+    - ``layout``: "auto" (two-phase edge-centric kernels for canonical edge lists of large
+      networks, else the fused kernel) or "fused";
     - ``kernel_timing``: bracket every kernel with CUDA events for ``Network.kernel_times``.
 
     The precision is the dtype given to ``adapt``.  The degree buckets (light rows up to 32,
@@ -369,7 +369,8 @@ class Network:
         capi.check(capi.load().nd_set_sum_order(self.handle, code))
 
     def set_layout(self, layout: str) -> None:
-        """'auto' (two-phase edge-centric kernels for canonical edge lists) or 'fused'."""
+        """'auto' (two-phase edge-centric kernels for canonical edge lists of large networks)
+        or 'fused'."""
         code = {"auto": 0, "fused": 1}[layout]
         capi.check(capi.load().nd_set_layout(self.handle, code))
 

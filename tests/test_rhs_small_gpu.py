@@ -1,0 +1,52 @@
+"""The RHS at the sizes where its kernels change: the fused launch of small networks and the
+two-phase layout above it, rows on both sides of the degree limits (a thread in a window, the
+heavy kernel or a block of the fused launch)."""
+import numpy as np
+import pytest
+
+import nd_gb300 as nd
+from oracle import oracle as O
+
+from ndtest import gpu_rhs, random_inputs
+
+pytestmark = pytest.mark.gpu
+
+VM = {O.V_DIFFUSION: nd.diffusion_vertex, O.V_SWING: nd.kuramoto_second}
+EM = {O.E_DIFFUSION: nd.diffusion_edge, O.E_KURAMOTO: nd.static_line}
+
+
+def hubs(degrees, nv):
+    """Vertices 0, 1, ... with the given degrees into the rest, and a path through the rest."""
+    k = len(degrees)
+    e = [(h, k + i) for h, d in enumerate(degrees) for i in range(d)] + [(i, i + 1) for i in range(k, nv - 1)]
+    arr = np.array(sorted(e), dtype=np.int64)
+    return nd.Graph(nv, np.ascontiguousarray(arr[:, 0]), np.ascontiguousarray(arr[:, 1]))
+
+
+@pytest.mark.parametrize("graph", [
+    lambda: nd.cycle_graph(3),                                  # one window
+    lambda: hubs([32, 33, 128, 129, 255, 256, 257], 700),       # fused: window / heavy rows
+    lambda: hubs([511, 512, 513, 1024, 1025, 2047, 2048, 2049, 2500], 6000),  # tiles of the block scan
+    lambda: nd.barabasi_albert(262_000, 4, seed=3),             # just below the FP64 fused limit
+    lambda: nd.barabasi_albert(263_000, 4, seed=3),             # just above it
+], ids=["cycle3", "hubs257", "hubs2500", "below", "above"])
+@pytest.mark.parametrize("vk,ek", [(O.V_DIFFUSION, O.E_DIFFUSION), (O.V_SWING, O.E_KURAMOTO)])
+def test_rhs_at_layout_limits(cuda, graph, vk, ek):
+    """Diffusion has the oracle's bits (no sine); with sines 1e-13 of the term scale, as the
+    other parity tests; FP32 within 4e-6 of it (24 eps of a compensated sum)."""
+    g = graph()
+    on = O.OracleNetwork.from_graph(g, vk, ek)
+    u, p = random_inputs(on, vk, np.random.default_rng(g.nv))
+    net = nd.Network(g, VM[vk](), EM[ek]())
+    import torch
+    got, ref = gpu_rhs(nd.adapt(net, torch.float64), u, p, cuda, np.float64), on.rhs(u, p)
+    scale = on.abs_terms(u, p) + np.abs(ref)
+    if ek == O.E_DIFFUSION:
+        np.testing.assert_array_equal(got, ref)
+    else:
+        assert np.all(np.abs(got - ref) <= 1e-13 * scale)
+    u32, p32 = u.astype(np.float32), p.astype(np.float32)
+    ref = on.rhs(u32.astype(np.float64), p32.astype(np.float64))
+    got = gpu_rhs(nd.adapt(net, torch.float32), u32, p32, cuda, np.float32)
+    scale = on.abs_terms(u32.astype(np.float64), p32.astype(np.float64)) + np.abs(ref)
+    assert np.all(np.abs(got - ref) <= 4e-6 * scale)
