@@ -172,6 +172,16 @@ __device__ __forceinline__ T thread_row_sum_deep(const T* __restrict__ y2, const
     T acc = T(0), comp = T(0);
     int ia[kB], ib[kB];
     T cur[kB], nxt[kB];
+    auto add = [&](T t) {  // 0 + t of the first term is the reference's zero start
+        if (kahan) {
+            const T yk = A::sub(t, comp);
+            const T s2 = A::add(acc, yk);
+            comp = A::sub(A::sub(s2, acc), yk);
+            acc = s2;
+        } else {
+            acc = A::add(acc, t);
+        }
+    };
     auto load_idx = [&](int j0, int (&ix)[kB]) {
 #pragma unroll
         for (int k = 0; k < kB; ++k) ix[k] = j0 + k < n ? __ldg(idx + j0 + k) : 0;
@@ -186,21 +196,17 @@ __device__ __forceinline__ T thread_row_sum_deep(const T* __restrict__ y2, const
     for (int j0 = 0; j0 < n; j0 += kB) {
         load_val(j0 + kB, ib, nxt);
         load_idx(j0 + 2 * kB, ia);
-        const int lim = __reduce_max_sync(__activemask(), (unsigned)min(kB, n - j0));
+        const unsigned lanes = __activemask();
+        if (__all_sync(lanes, j0 + kB <= n)) {
+            // every row of the warp has the whole batch: nothing between the dependent adds
 #pragma unroll
-        for (int k = 0; k < kB; ++k) {
-            if (k >= lim) break;
-            if (j0 + k >= n) continue;
-            if (sizeof(T) == 8 && j0 + k == 0) {
-                const double t0 = (double)cur[0];
-                acc = (T)((__double_as_longlong(t0) << 1) == 0 ? 0.0 : t0);
-            } else if (kahan) {
-                const T yk = A::sub(cur[k], comp);
-                const T s2 = A::add(acc, yk);
-                comp = A::sub(A::sub(s2, acc), yk);
-                acc = s2;
-            } else {
-                acc = A::add(acc, cur[k]);
+            for (int k = 0; k < kB; ++k) add(cur[k]);
+        } else {
+            const int lim = __reduce_max_sync(lanes, (unsigned)min(kB, n - j0));
+#pragma unroll
+            for (int k = 0; k < kB; ++k) {
+                if (k >= lim) break;
+                if (j0 + k < n) add(cur[k]);
             }
         }
 #pragma unroll

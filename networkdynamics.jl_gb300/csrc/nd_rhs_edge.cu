@@ -297,11 +297,18 @@ __device__ __forceinline__ void pipelined_sum(int n, Load&& load, Add&& add) {
     load(0, cur);
     for (int j0 = 0; j0 < n; j0 += KB) {
         load(j0 + KB, nxt);
-        const int lim = __reduce_max_sync(__activemask(), (unsigned)min(KB, n - j0));
+        const unsigned lanes = __activemask();
+        if (__all_sync(lanes, j0 + KB <= n)) {
+            // every row of the warp has the whole batch: nothing between the dependent adds
 #pragma unroll
-        for (int k = 0; k < KB; ++k) {
-            if (k >= lim) break;
-            if (j0 + k < n) add(j0 + k, cur[k]);
+            for (int k = 0; k < KB; ++k) add(cur[k]);
+        } else {
+            const int lim = __reduce_max_sync(lanes, (unsigned)min(KB, n - j0));
+#pragma unroll
+            for (int k = 0; k < KB; ++k) {
+                if (k >= lim) break;
+                if (j0 + k < n) add(cur[k]);
+            }
         }
 #pragma unroll
         for (int k = 0; k < KB; ++k) cur[k] = nxt[k];
@@ -358,13 +365,9 @@ __global__ void __launch_bounds__(kDenseBlock) dense_row_kernel(RhsArgs a) {
                 for (int k = 0; k < KB; ++k) t[k] = j0 + k < nd ? ld_hint(ybkt + pos[k], stream) : T(0);
                 load_pos(j0 + KB);  // the positions of the batch after
             },
-            [&](int j, T t) {
-                if constexpr (sizeof(T) == 8) {
-                    if (j == 0) acc = (T)((__double_as_longlong((double)t) << 1) == 0 ? 0.0 : (double)t);
-                    else acc = __dadd_rn(acc, t);
-                } else {
-                    add(t);
-                }
+            [&](T t) {  // 0 + t of the first term is the reference's zero start
+                if constexpr (sizeof(T) == 8) acc = __dadd_rn(acc, t);
+                else add(t);
             });
     }
     // source side: the row's own block of y
@@ -374,7 +377,7 @@ __global__ void __launch_bounds__(kDenseBlock) dense_row_kernel(RhsArgs a) {
 #pragma unroll
             for (int k = 0; k < KB; ++k) t[k] = j0 + k < ns ? ld_hint(y + sp + (uint32_t)(j0 + k), stream) : T(0);
         },
-        [&](int, T t) {
+        [&](T t) {
             if constexpr (sizeof(T) == 8) acc = __dsub_rn(acc, t);
             else add(-t);
         });
