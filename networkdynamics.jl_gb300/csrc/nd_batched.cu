@@ -55,9 +55,12 @@ struct BatchedKArgs {
     BatchTableDev vb, eb;  // the batch tables (device arrays)
     const int2* eu;
     const uint32_t* tptr;
-    const int32_t* tidx;
     const int32_t* slot_vpos;
     void* y2;
+    // what the rows sum: y2 by the terms' y2 indices, or u by the terms' edge states (see
+    // BatchedNet::tstate)
+    const void* row_vals;
+    const int32_t* tidx;
     int32_t mode;
 };
 
@@ -75,7 +78,9 @@ __global__ void __launch_bounds__(kBlock) batched_edge_kernel(BatchedKArgs a) {
     const T* __restrict__ u = static_cast<const T*>(a.u);
     const T* __restrict__ p = static_cast<const T*>(a.p);
     T* __restrict__ du = static_cast<T*>(a.du);
-    V2* __restrict__ y2 = static_cast<V2*>(a.y2);
+    V2* __restrict__ y2 = a.row_vals == a.y2 ? static_cast<V2*>(a.y2) : nullptr;
+    // edge state pairs as vectors, where the caller's buffers allow it
+    const bool pairs = (reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(du)) % sizeof(V2) == 0;
     for (int64_t k = (int64_t)blockIdx.x * kBlock + threadIdx.x; k < a.ne; k += (int64_t)gridDim.x * kBlock) {
         const int b = find_batch(a.eb, k);
         const int kind = __ldg(a.eb.kind + b);
@@ -85,14 +90,24 @@ __global__ void __launch_bounds__(kBlock) batched_edge_kernel(BatchedKArgs a) {
         V2 y;
         if (kind == ND_E_DIFFUSION_ODE || kind == ND_E_DIFFUSION_ODE_FIXED) {
             const int64_t s = __ldg(a.eb.s0 + b) + 2 * r;
-            const T e1 = __ldg(u + s), e2 = __ldg(u + s + 1);
+            const bool vec = pairs && !(s & 1);
+            V2 e, d;
+            if (vec) {
+                e = __ldg(reinterpret_cast<const V2*>(u + s));
+            } else {
+                e.x = __ldg(u + s);
+                e.y = __ldg(u + s + 1);
+            }
             const T rate = kind == ND_E_DIFFUSION_ODE ? A::div(T(1), __ldg(p + __ldg(a.eb.p0 + b) + r)) : T(100);
-            T d1, d2;
-            ode_edge_f<T>(rate, vs, vd, e1, e2, d1, d2);
-            du[s] = d1;
-            du[s + 1] = d2;
-            y.x = e2;  // Fiducial(dst=1:1, src=2:2): y_src = e2, y_dst = e1
-            y.y = e1;
+            ode_edge_f<T>(rate, vs, vd, e.x, e.y, d.x, d.y);
+            if (vec) {
+                *reinterpret_cast<V2*>(du + s) = d;
+            } else {
+                du[s] = d.x;
+                du[s + 1] = d.y;
+            }
+            y.x = e.y;  // Fiducial(dst=1:1, src=2:2): y_src = e2, y_dst = e1
+            y.y = e.x;
         } else {
             const T w = kind == ND_E_DIFFUSION_UNIT ? T(0) : __ldg(p + __ldg(a.eb.p0 + b) + r);
             const T yd = static_edge_g<T>(kind, vs, vd, w);
@@ -102,7 +117,7 @@ __global__ void __launch_bounds__(kBlock) batched_edge_kernel(BatchedKArgs a) {
             y.x = c == ND_SYMMETRIC ? yd : (c == ND_DIRECTED ? T(0) : -yd);
             y.y = yd;
         }
-        y2[k] = y;
+        if (y2) y2[k] = y;  // not where the rows read the edge states themselves
     }
 }
 
@@ -310,7 +325,7 @@ constexpr int kRowBlock = 64;
 template <typename T, bool kDense, int NT>
 __global__ void __launch_bounds__(NT) batched_row_kernel(BatchedKArgs a, int64_t n_warp_blocks) {
     constexpr int kWarps = NT / 32;
-    const T* __restrict__ y2 = static_cast<const T*>(a.y2);
+    const T* __restrict__ y2 = static_cast<const T*>(a.row_vals);
     if ((int64_t)blockIdx.x < n_warp_blocks) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const int64_t slot = (int64_t)blockIdx.x * kWarps + warp;
@@ -417,9 +432,10 @@ cudaError_t launch_typed(const BatchedNet& b, void* du, const void* u, const voi
     a.eb = b.deb;
     a.eu = b.eu;
     a.tptr = b.tptr;
-    a.tidx = b.tidx;
+    a.tidx = b.tstate ? b.tstate : b.tidx;
     a.slot_vpos = b.slot_vpos;
     a.y2 = b.y2;
+    a.row_vals = b.tstate ? u : b.y2;
     a.mode = mode;
     if (b.depth == 2) {
         if ((phases & kPhaseEdge) && b.ne > 0) {
@@ -510,6 +526,7 @@ void free_batched(BatchedNet* b) {
     cudaFree(b->eu);
     cudaFree(b->tptr);
     cudaFree(b->tidx);
+    cudaFree(b->tstate);
     cudaFree(b->slot_vpos);
     cudaFree(b->y2);
     *b = BatchedNet{};
@@ -716,6 +733,18 @@ int build_batched(const nd_batched_network_desc* d, int elem, BatchedNet* out) {
         for (int32_t v : shortr) (deg[v] > (uint32_t)kLightMaxDeg ? inc_long : inc_short) += deg[v];
         bn.dense_rows = elem == 8 && inc_long > inc_short;
     }
+    // networks of ODE edges only: every term is a state of the caller's u
+    std::vector<int32_t> tstate;
+    bool all_ode = elem > 0 && ne > 0;
+    for (int b = 0; b < neb; ++b) all_ode = all_ode && (ode_kind(eb.kind[b]) || ecount[b] == 0);
+    if (all_ode) {
+        // states of edge position k: (e1, e2), y_dst = e1 (term 2k + 1), y_src = e2 (term 2k)
+        std::vector<int32_t> first(ne);
+        for (int b = 0; b < neb; ++b)
+            for (int64_t k = eb.pos0[b]; k < eb.pos0[b + 1]; ++k) first[k] = (int32_t)(eb.s0[b] + 2 * (k - eb.pos0[b]));
+        tstate.resize((size_t)2 * ne);
+        for (size_t j = 0; j < tstate.size(); ++j) tstate[j] = first[tidx[j] >> 1] + ((tidx[j] & 1) ? 0 : 1);
+    }
     auto upload = [&](void** dptr, const void* hptr, size_t bytes) -> cudaError_t {
         cudaError_t err = cudaMalloc(dptr, std::max<size_t>(bytes, 16));
         if (err != cudaSuccess) return err;
@@ -728,7 +757,9 @@ int build_batched(const nd_batched_network_desc* d, int elem, BatchedNet* out) {
         (err = upload((void**)&bn.tptr, tptr.data(), tptr.size() * sizeof(uint32_t))) != cudaSuccess ||
         (err = upload((void**)&bn.tidx, tidx.data(), tidx.size() * sizeof(int32_t))) != cudaSuccess ||
         (err = upload((void**)&bn.slot_vpos, slot_vpos.data(), slot_vpos.size() * sizeof(int32_t))) != cudaSuccess ||
-        (elem > 0 && (err = cudaMalloc(&bn.y2, std::max<size_t>((size_t)2 * depth * ne * elem, 16))) != cudaSuccess)) {
+        (all_ode && (err = upload((void**)&bn.tstate, tstate.data(), tstate.size() * sizeof(int32_t))) != cudaSuccess) ||
+        (elem > 0 && !all_ode &&
+         (err = cudaMalloc(&bn.y2, std::max<size_t>((size_t)2 * depth * ne * elem, 16))) != cudaSuccess)) {
         free_batched(&bn);
         return cuda_fail(err, "upload of the batched network");
     }

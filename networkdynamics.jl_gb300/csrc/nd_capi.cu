@@ -581,12 +581,23 @@ int nd_rhs(nd_handle* h, int dtype, void* du, int64_t n_du, const void* u, int64
     if (h->batched.enabled) {
         const BatchedNet& b = h->batched;
         cudaError_t err = cudaSuccess;
-        if (b.ne > 0)
+        // rows that read only u (ODE edges) run beside the edges, forked and joined by events
+        const bool beside = b.tstate && h->dtype == ND_F32 && b.ne >= kOverlapRowsMinEdges;
+        const cudaStream_t rs = beside ? h->side : s;
+        if (beside && ((err = cudaEventRecord(h->ev_fork, s)) != cudaSuccess ||
+                       (err = cudaStreamWaitEvent(rs, h->ev_fork, 0)) != cudaSuccess))
+            return cuda_fail(err, "nd_rhs kernel launch");
+        auto rows = [&] {
+            return traced(h, kKernelBatchedRows, rs,
+                          [&] { return launch_batched(h->dtype, b, du, u, p, h->rhs_mode, rs, kPhaseRow); });
+        };
+        if (beside) err = rows();
+        if (err == cudaSuccess && b.ne > 0)
             err = traced(h, kKernelBatchedEdges, s,
                          [&] { return launch_batched(h->dtype, b, du, u, p, h->rhs_mode, s, kPhaseEdge); });
-        if (err == cudaSuccess)
-            err = traced(h, kKernelBatchedRows, s,
-                         [&] { return launch_batched(h->dtype, b, du, u, p, h->rhs_mode, s, kPhaseRow); });
+        if (err == cudaSuccess && !beside) err = rows();
+        if (err == cudaSuccess && beside && (err = cudaEventRecord(h->ev_join, rs)) == cudaSuccess)
+            err = cudaStreamWaitEvent(s, h->ev_join, 0);
         return err == cudaSuccess ? ND_OK : cuda_fail(err, "nd_rhs kernel launch");
     }
     RhsArgs a;

@@ -216,6 +216,12 @@ struct RhsArgs {
 // Launch the fused RHS for the given element type.
 cudaError_t launch_rhs(int dtype, const RhsArgs& a, cudaStream_t stream);
 // Launch the two-phase (edge-centric) RHS: phase E, phase R or both (kPhase* bits).
+// FP32 rows of ODE-edge networks with at least this many edges run on the handle's side stream
+// beside the edge kernel (WS(3000, 1500): 28.8 µs one after the other, 23.5 beside; WS(1500, 750)
+// 14.4 and 11.2).  Below, the four event calls cost more than the shorter kernel.  Not in FP64,
+// where the rows' chains of adds then wait for the edges' operations in the SM's one FP64 unit
+// (109 µs one after the other, 172 beside).
+constexpr int64_t kOverlapRowsMinEdges = 200000;
 enum : int { kPhaseEdge = 1, kPhaseRow = 2, kPhaseBoth = 3 };
 cudaError_t launch_rhs_edge(int dtype, const RhsArgs& a, cudaStream_t stream, int phases = kPhaseBoth);
 
@@ -277,6 +283,9 @@ struct BatchedNet {
     int2* eu = nullptr;          // [ne] by edge position: u indices of the src / dst vertex outputs
     uint32_t* tptr = nullptr;    // [nv+1] by slot: range of the slot's terms in tidx
     int32_t* tidx = nullptr;     // [2ne] y2 indices of every row's terms, ascending
+    // networks of ODE edges only: the u index of every term, in tidx's order (such an edge's outputs
+    // are its states, so the rows read u and need nothing from the edge kernel); y2 is not used
+    int32_t* tstate = nullptr;   // [2ne]
     int32_t* slot_vpos = nullptr;  // [nv] vertex position of each slot
     void* y2 = nullptr;          // [2ne·depth] scratch, element type of the handle
 };
