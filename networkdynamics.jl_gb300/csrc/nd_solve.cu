@@ -4,8 +4,8 @@
 // The state, the stage vectors, the error norm and the step controller are FP64 on the
 // device; the RHS runs in the handle's precision (an FP32 handle converts each stage
 // state to FP32 and the stage derivative back).  Stage combinations use the operation
-// order of the CPU oracle's Tsit5 (acc = Σ_j a_sj·k_j left to right, y = u + h·acc, no
-// fused multiply-adds).  Step control stays on the device: the step size, the time and
+// order of the CPU oracle's Tsit5 (acc = Σ_j a_sj·k_j left to right, y = u + h·acc), as fused
+// multiply-adds.  Step control stays on the device: the step size, the time and
 // the accept flag live in device memory, so the host enqueues steps without waiting; one
 // step is captured into a CUDA graph and replayed, and the host reads the status every
 // few steps.
@@ -14,6 +14,7 @@
 #include <cstring>
 #include <vector>
 
+#include "nd_exact.cuh"
 #include "nd_internal.h"
 
 namespace nd {
@@ -26,7 +27,6 @@ constexpr int kSB = 256;
 __constant__ double c_a[7][6];
 __constant__ double c_bt[7];
 
-const double h_c[7] = {0.0, 0.161, 0.327, 0.9, 0.9800255409045097, 1.0, 1.0};
 const double h_a[7][6] = {
     {0, 0, 0, 0, 0, 0},
     {0.161, 0, 0, 0, 0, 0},
@@ -39,6 +39,11 @@ const double h_bt[7] = {-0.00178001105222577714, -0.0008164344596567469, 0.00788
                         -0.1447110071732629,     0.5823571654525552,     -0.45808210592918697,
                         0.015151515151515152};
 
+// The stage derivatives, by value (a kernel argument).
+struct Stages {
+    double* k[7];
+};
+
 // Controller state in device memory.
 struct Ctl {
     double t, t1, dt, qold, eest;
@@ -49,14 +54,30 @@ struct Ctl {
     int accept;  // last step accepted
 };
 
-__global__ void stage_kernel(int s, int64_t n, const double* __restrict__ u, double* const* __restrict__ k,
-                             double* __restrict__ y, const Ctl* ctl) {
+// y = u + h Σ_j a_sj k_j by fused multiply-adds (S + 1 FP64 operations an entry, which bound it; 2 S + 2
+// as separate products and sums).
+template <int S>
+__global__ void __launch_bounds__(kSB) stage_kernel(int64_t n, const double* __restrict__ u, Stages k,
+                                                    double* __restrict__ y, const Ctl* ctl) {
     if (ctl->done) return;
     const double h = ctl->dt;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double acc = 0.0;
-        for (int j = 0; j < s; ++j) acc = __dadd_rn(acc, __dmul_rn(c_a[s][j], k[j][i]));
-        y[i] = __dadd_rn(u[i], __dmul_rn(h, acc));
+    for (int64_t i = (int64_t)blockIdx.x * kSB + threadIdx.x; i < n; i += (int64_t)gridDim.x * kSB) {
+        double acc = __dmul_rn(c_a[S][0], k.k[0][i]);
+#pragma unroll
+        for (int j = 1; j < S; ++j) acc = __fma_rn(c_a[S][j], k.k[j][i], acc);
+        y[i] = __fma_rn(h, acc, u[i]);
+    }
+}
+
+void launch_stage(int st, unsigned g, int64_t n, const double* u, const Stages& k, double* y, const Ctl* ctl,
+                  cudaStream_t s) {
+    switch (st) {
+        case 1: stage_kernel<1><<<g, kSB, 0, s>>>(n, u, k, y, ctl); break;
+        case 2: stage_kernel<2><<<g, kSB, 0, s>>>(n, u, k, y, ctl); break;
+        case 3: stage_kernel<3><<<g, kSB, 0, s>>>(n, u, k, y, ctl); break;
+        case 4: stage_kernel<4><<<g, kSB, 0, s>>>(n, u, k, y, ctl); break;
+        case 5: stage_kernel<5><<<g, kSB, 0, s>>>(n, u, k, y, ctl); break;
+        default: stage_kernel<6><<<g, kSB, 0, s>>>(n, u, k, y, ctl);
     }
 }
 
@@ -71,36 +92,89 @@ __global__ void to_f64_kernel(int64_t n, const float* __restrict__ x, double* __
         y[i] = (double)x[i];
 }
 
-// Per-block partial sums of ((h Σ btilde_j k_j) / (abstol + reltol max(|u|,|y|)))^2, fixed order.
-__global__ void error_kernel(int64_t n, const double* __restrict__ u, const double* __restrict__ ynew,
-                             double* const* __restrict__ k, double* __restrict__ partial, const Ctl* ctl) {
+// Sum of one value per thread over the block, in a fixed order; the result is in thread 0.
+__device__ __forceinline__ double block_total(double s) {
     __shared__ double red[kSB];
-    double s = 0.0;
-    if (!ctl->done) {
-        const double h = ctl->dt;
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-            double acc = 0.0;
-            for (int j = 0; j < 7; ++j) acc = __dadd_rn(acc, __dmul_rn(c_bt[j], k[j][i]));
-            const double e = __dmul_rn(h, acc);
-            const double sc = ctl->abstol + ctl->reltol * fmax(fabs(u[i]), fabs(ynew[i]));
-            const double r = e / sc;
-            s += r * r;
-        }
-    }
+    __syncthreads();
     red[threadIdx.x] = s;
     __syncthreads();
-    for (int off = kSB / 2; off > 0; off >>= 1) {
-        if ((int)threadIdx.x < off) red[threadIdx.x] += red[threadIdx.x + off];
-        __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x < 32) {
+#pragma unroll
+        for (int j = 0; j < kSB / 32; ++j) t += red[threadIdx.x + 32 * j];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
     }
-    if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
+    return t;
 }
 
-// Step-size control (PI controller, the oracle's constants) on one thread.
-__global__ void control_kernel(int nblocks, int64_t n, const double* __restrict__ partial, Ctl* ctl) {
-    if (threadIdx.x != 0 || blockIdx.x != 0 || ctl->done) return;
+// Per-block partial sums of ((h Σ btilde_j k_j) / (abstol + reltol max(|u|,|y|)))^2, fixed order.
+__global__ void __launch_bounds__(kSB) error_kernel(int64_t n, const double* __restrict__ u,
+                                                    const double* __restrict__ ynew, Stages k,
+                                                    double* __restrict__ partial, const Ctl* ctl) {
     double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) s += partial[b];
+    if (!ctl->done) {
+        const double h = ctl->dt, reltol = ctl->reltol, abstol = ctl->abstol;
+        for (int64_t i = (int64_t)blockIdx.x * kSB + threadIdx.x; i < n; i += (int64_t)gridDim.x * kSB) {
+            double acc = __dmul_rn(c_bt[0], k.k[0][i]);
+#pragma unroll
+            for (int j = 1; j < 7; ++j) acc = __fma_rn(c_bt[j], k.k[j][i], acc);
+            const double sc = __fma_rn(reltol, fmax(fabs(u[i]), fabs(ynew[i])), abstol);
+            const double r = exact::div_rn(__dmul_rn(h, acc), sc);
+            s = __fma_rn(r, r, s);
+        }
+    }
+    s = block_total(s);
+    if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+
+// The initial step's norms: per-block partial sums of (u / sc)^2 and (a / sc)^2 (with b: of
+// ((a - b) / sc)^2 only), sc = abstol + |u| reltol.
+__global__ void __launch_bounds__(kSB) norm_kernel(int64_t n, const double* __restrict__ u, const double* __restrict__ a,
+                                                   const double* __restrict__ b, double* __restrict__ partial,
+                                                   const Ctl* ctl) {
+    double s0 = 0.0, s1 = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * kSB + threadIdx.x; i < n; i += (int64_t)gridDim.x * kSB) {
+        const double sc = ctl->abstol + fabs(u[i]) * ctl->reltol;
+        const double r0 = b ? 0.0 : exact::div_rn(u[i], sc), r1 = exact::div_rn(b ? a[i] - b[i] : a[i], sc);
+        s0 += r0 * r0;
+        s1 += r1 * r1;
+    }
+    s0 = block_total(s0);
+    s1 = block_total(s1);
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = s0;
+        partial[gridDim.x + blockIdx.x] = s1;
+    }
+}
+
+// out[j] = Σ of the j-th set of nblocks partials, a block per set.
+__global__ void __launch_bounds__(kSB) total_kernel(int nblocks, const double* __restrict__ partial,
+                                                    double* __restrict__ out) {
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nblocks; b += kSB) s += partial[(int64_t)blockIdx.x * nblocks + b];
+    s = block_total(s);
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
+}
+
+__global__ void __launch_bounds__(kSB) euler_kernel(int64_t n, double h, const double* __restrict__ u,
+                                                    const double* __restrict__ k, double* __restrict__ y) {
+    for (int64_t i = (int64_t)blockIdx.x * kSB + threadIdx.x; i < n; i += (int64_t)gridDim.x * kSB) y[i] = u[i] + h * k[i];
+}
+
+// Step-size control (PI controller, the oracle's constants): one block adds the partials (one
+// thread took 33 µs for the 782 of 2e5 states), its first thread decides.  A step after the end
+// of the solve only leaves its mark.
+__global__ void __launch_bounds__(kSB) control_kernel(int nblocks, int64_t n, const double* __restrict__ partial, Ctl* ctl,
+                                                      int* last_seen) {
+    if (ctl->done) {
+        if (threadIdx.x == 0) *last_seen = 1;
+        return;
+    }
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nblocks; b += kSB) s += partial[b];
+    s = block_total(s);
+    if (threadIdx.x != 0) return;
     double EEst = sqrt(s / (double)(n > 0 ? n : 1));
     if (!(EEst == EEst)) EEst = 1e10;
     const double beta1 = 7.0 / 50.0, beta2 = 2.0 / 25.0, gamma = 0.9, qmin = 0.2, qmax = 10.0;
@@ -146,15 +220,10 @@ __global__ void accept_kernel(int64_t n, double* __restrict__ u, const double* _
         k0[i] = k6[i];
     }
 }
-__global__ void mark_kernel(const Ctl* ctl, int* last_seen) {
-    if (threadIdx.x == 0 && blockIdx.x == 0 && ctl->done) *last_seen = 1;
-}
-
 struct Workspace {
     int64_t n = 0;
-    double* k[7] = {};
+    Stages st = {};
     double* y = nullptr;
-    double** kptr = nullptr;
     float* y32 = nullptr;
     float* k32 = nullptr;
     double* partial = nullptr;
@@ -164,9 +233,8 @@ struct Workspace {
 };
 
 void free_ws(Workspace& w) {
-    for (auto& p : w.k) cudaFree(p);
+    for (auto& p : w.st.k) cudaFree(p);
     cudaFree(w.y);
-    cudaFree(w.kptr);
     cudaFree(w.y32);
     cudaFree(w.k32);
     cudaFree(w.partial);
@@ -241,21 +309,18 @@ extern "C" int nd_solve_tsit5(nd_handle* h, double* u, const void* p, double t0,
             return rc;                                   \
         }                                                \
     } while (0)
-    for (auto& k : w.k) ND_WS(cudaMalloc(&k, sizeof(double) * std::max<int64_t>(n, 1)));
+    for (auto& k : w.st.k) ND_WS(cudaMalloc(&k, sizeof(double) * std::max<int64_t>(n, 1)));
     ND_WS(cudaMalloc(&w.y, sizeof(double) * std::max<int64_t>(n, 1)));
-    ND_WS(cudaMalloc(&w.kptr, sizeof(double*) * 7));
-    ND_WS(cudaMemcpy(w.kptr, w.k, sizeof(double*) * 7, cudaMemcpyHostToDevice));
     if (h->dtype == ND_F32) {
         ND_WS(cudaMalloc(&w.y32, sizeof(float) * std::max<int64_t>(n, 1)));
         ND_WS(cudaMalloc(&w.k32, sizeof(float) * std::max<int64_t>(n, 1)));
     }
-    ND_WS(cudaMalloc(&w.partial, sizeof(double) * w.nblocks));
+    ND_WS(cudaMalloc(&w.partial, sizeof(double) * (2 * (size_t)w.nblocks + 2)));
     ND_WS(cudaMalloc(&w.ctl, sizeof(Ctl)));
     ND_WS(cudaMalloc(&w.last_seen, sizeof(int)));
     ND_WS(cudaMemsetAsync(w.last_seen, 0, sizeof(int), s));
 
-    // Initial step (Hairer & Wanner, order 5), on the host from two RHS evaluations.
-    std::vector<double> hu(n), hk0(n), hk1(n);
+    // Initial step (Hairer & Wanner, order 5) from the norms of two RHS evaluations.
     Ctl c{};
     c.t = t0;
     c.t1 = t1;
@@ -266,39 +331,32 @@ extern "C" int nd_solve_tsit5(nd_handle* h, double* u, const void* p, double t0,
     c.done = 0;
     c.status = ND_OK;
     ND_WS(cudaMemcpyAsync(w.ctl, &c, sizeof c, cudaMemcpyHostToDevice, s));
-    if ((rc = rhs_f64(h, w, w.k[0], u, p, nullptr, s)) != ND_OK) {
+    double* totals = w.partial + 2 * (size_t)w.nblocks;
+    double d01[2] = {0.0, 0.0};
+    // d01 <- square roots of the two mean sums of norm_kernel(a, b)
+    auto norms = [&](const double* a, const double* b) -> cudaError_t {
+        norm_kernel<<<g, kSB, 0, s>>>(n, u, a, b, w.partial, w.ctl);
+        total_kernel<<<2, kSB, 0, s>>>(w.nblocks, w.partial, totals);
+        cudaError_t e = cudaMemcpyAsync(d01, totals, sizeof d01, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        for (double& d : d01) d = sqrt(d / (double)(n ? n : 1));
+        return e;
+    };
+    if ((rc = rhs_f64(h, w, w.st.k[0], u, p, nullptr, s)) != ND_OK) {
         cleanup();
         return rc;
     }
-    ND_WS(cudaMemcpyAsync(hu.data(), u, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-    ND_WS(cudaMemcpyAsync(hk0.data(), w.k[0], sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-    ND_WS(cudaStreamSynchronize(s));
-    double d0 = 0, d1 = 0;
-    for (int64_t i = 0; i < n; ++i) {
-        const double sc = abstol + fabs(hu[i]) * reltol;
-        d0 += (hu[i] / sc) * (hu[i] / sc);
-        d1 += (hk0[i] / sc) * (hk0[i] / sc);
-    }
-    d0 = sqrt(d0 / (double)(n ? n : 1));
-    d1 = sqrt(d1 / (double)(n ? n : 1));
+    ND_WS(norms(w.st.k[0], nullptr));
+    const double d0 = d01[0], d1 = d01[1];
     double h0 = (d0 < 1e-5 || d1 < 1e-5) ? 1e-6 : 0.01 * (d0 / d1);
     h0 = fmin(h0, t1 - t0);
-    std::vector<double> hy(n);
-    for (int64_t i = 0; i < n; ++i) hy[i] = hu[i] + h0 * hk0[i];
-    ND_WS(cudaMemcpyAsync(w.y, hy.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    if ((rc = rhs_f64(h, w, w.k[1], w.y, p, nullptr, s)) != ND_OK) {
+    euler_kernel<<<g, kSB, 0, s>>>(n, h0, u, w.st.k[0], w.y);
+    if ((rc = rhs_f64(h, w, w.st.k[1], w.y, p, nullptr, s)) != ND_OK) {
         cleanup();
         return rc;
     }
-    ND_WS(cudaMemcpyAsync(hk1.data(), w.k[1], sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-    ND_WS(cudaStreamSynchronize(s));
-    double d2 = 0;
-    for (int64_t i = 0; i < n; ++i) {
-        const double sc = abstol + fabs(hu[i]) * reltol;
-        const double r = (hk1[i] - hk0[i]) / sc;
-        d2 += r * r;
-    }
-    d2 = sqrt(d2 / (double)(n ? n : 1)) / h0;
+    ND_WS(norms(w.st.k[1], w.st.k[0]));
+    const double d2 = d01[1] / h0;
     const double h1 = (fmax(d1, d2) <= 1e-15) ? fmax(1e-6, h0 * 1e-3) : pow(0.01 / fmax(d1, d2), 1.0 / 5.0);
     c.dt = fmin(fmin(100 * h0, h1), t1 - t0);
     ND_WS(cudaMemcpyAsync(w.ctl, &c, sizeof c, cudaMemcpyHostToDevice, s));
@@ -311,13 +369,12 @@ extern "C" int nd_solve_tsit5(nd_handle* h, double* u, const void* p, double t0,
     ND_WS(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     bool ok = true;
     for (int st = 1; st < 7 && ok; ++st) {
-        stage_kernel<<<g, kSB, 0, s>>>(st, n, u, w.kptr, w.y, w.ctl);
-        ok = rhs_f64(h, w, w.k[st], w.y, p, w.ctl, s) == ND_OK;
+        launch_stage(st, g, n, u, w.st, w.y, w.ctl, s);
+        ok = rhs_f64(h, w, w.st.k[st], w.y, p, w.ctl, s) == ND_OK;
     }
-    error_kernel<<<g, kSB, 0, s>>>(n, u, w.y, w.kptr, w.partial, w.ctl);
-    mark_kernel<<<1, 32, 0, s>>>(w.ctl, w.last_seen);
-    control_kernel<<<1, 32, 0, s>>>(w.nblocks, n, w.partial, w.ctl);
-    accept_kernel<<<g, kSB, 0, s>>>(n, u, w.y, w.k[0], w.k[6], w.ctl, w.last_seen);
+    error_kernel<<<g, kSB, 0, s>>>(n, u, w.y, w.st, w.partial, w.ctl);
+    control_kernel<<<1, kSB, 0, s>>>(w.nblocks, n, w.partial, w.ctl, w.last_seen);
+    accept_kernel<<<g, kSB, 0, s>>>(n, u, w.y, w.st.k[0], w.st.k[6], w.ctl, w.last_seen);
     cudaError_t cap = cudaStreamEndCapture(s, &graph);
     if (!ok) {
         if (graph) cudaGraphDestroy(graph);
@@ -327,9 +384,12 @@ extern "C" int nd_solve_tsit5(nd_handle* h, double* u, const void* p, double t0,
     }
     ND_WS(cap);
     ND_WS(cudaGraphInstantiate(&exec, graph, 0));
-    const int kBatch = 16;
+    // up to 16 steps between two looks at the status, fewer where the step size says that fewer are
+    // left: a replay after the end still evaluates its six right-hand sides
     for (;;) {
-        for (int i = 0; i < kBatch; ++i) ND_WS(cudaGraphLaunch(exec, s));
+        const double left = (c.t1 - c.t) / c.dt;
+        const int batch = left < 15.0 ? std::max(1, (int)std::ceil(left)) : 16;  // NaN: 16
+        for (int i = 0; i < batch; ++i) ND_WS(cudaGraphLaunch(exec, s));
         ND_WS(cudaMemcpyAsync(&c, w.ctl, sizeof c, cudaMemcpyDeviceToHost, s));
         ND_WS(cudaStreamSynchronize(s));
         if (c.done) break;
