@@ -65,7 +65,8 @@ struct EdgeLayoutHost {
     int64_t n_chunks = 0;
 };
 
-static void build_edge_layout(int64_t nv, int64_t ne, const int64_t* src, const int64_t* dst, EdgeLayoutHost& h) {
+static void build_edge_layout(int64_t nv, int64_t ne, const int64_t* src, const int64_t* dst, bool direct,
+                              EdgeLayoutHost& h) {
     h.esrc.resize(ne);
     h.edst.resize(ne);
     h.dptr.assign(nv + 1, 0);
@@ -85,6 +86,12 @@ static void build_edge_layout(int64_t nv, int64_t ne, const int64_t* src, const 
     {
         std::vector<uint32_t> fill(h.dptr.begin(), h.dptr.end() - 1);
         for (int64_t e = 0; e < ne; ++e) tpos[e] = fill[dst[e]]++;
+    }
+    h.loc.resize(ne);
+    if (direct) {  // the rows read y itself
+        h.n_chunks = (ne + kDirectChunk - 1) / kDirectChunk;
+        for (int64_t e = 0; e < ne; ++e) h.loc[tpos[e]] = (int32_t)e;
+        return;
     }
     // buckets of destination-CSR positions; ybkt is bucket-major, chunk-major inside a
     // bucket, edge order inside a (bucket, chunk) run
@@ -112,7 +119,6 @@ static void build_edge_layout(int64_t nv, int64_t ne, const int64_t* src, const 
     for (int64_t c = 0; c < nch; ++c)
         for (int b = 0; b < kBuckets; ++b) h.run_base[c * kBuckets + b] = (int32_t)cnt[(size_t)b * nch + c];
     h.lslot.resize(ne);
-    h.loc.resize(ne);
     for (int64_t e = 0; e < ne; ++e) {
         const size_t key = (size_t)(tpos[e] / bsize) * nch + e / kEdgeChunk;
         const int64_t qe = cnt[key]++;
@@ -267,7 +273,8 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
     }
     if (canonical && !small) {
         EdgeLayoutHost h;
-        build_edge_layout(nv, ne, src, dst, h);
+        const bool direct = ne * edge_elem <= kDirectMaxBytes;
+        build_edge_layout(nv, ne, src, dst, direct, h);
         // the row records and the padded loc array, in slot order of the rows
         std::vector<int64_t> lstart(nv + 1, 0);
         for (int64_t v = 0; v < nv; ++v) lstart[v + 1] = lstart[v] + ((h.dptr[v + 1] - h.dptr[v] + 3) & ~3u);
@@ -286,6 +293,7 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
         }
         EdgeLayout& el = t.edge;
         el.n_chunks = h.n_chunks;
+        el.direct = direct;
         if ((err = upload((void**)&el.esrc, h.esrc.data(), h.esrc.size() * sizeof(int32_t))) != cudaSuccess ||
             (err = upload((void**)&el.edst, h.edst.data(), h.edst.size() * sizeof(int32_t))) != cudaSuccess ||
             (err = upload((void**)&el.lslot, h.lslot.data(), h.lslot.size() * sizeof(uint16_t))) != cudaSuccess ||
@@ -297,7 +305,7 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
             (err = upload((void**)&el.locp, locp.data(), locp.size() * sizeof(int32_t))) != cudaSuccess ||
             (err = cudaMalloc(&el.y, (size_t)(ne + 2) * edge_elem)) != cudaSuccess ||
             (err = cudaMemset(el.y, 0, (size_t)(ne + 2) * edge_elem)) != cudaSuccess ||
-            (err = cudaMalloc(&el.ybkt, (size_t)ne * edge_elem)) != cudaSuccess) {
+            (!direct && (err = cudaMalloc(&el.ybkt, (size_t)ne * edge_elem)) != cudaSuccess)) {
             free_topology(&t);
             return cuda_fail(err, "upload of the edge-centric layout");
         }
@@ -627,7 +635,8 @@ int nd_rhs(nd_handle* h, int dtype, void* du, int64_t n_du, const void* u, int64
     a.rmeta = el.rmeta;
     a.locp = el.locp;
     a.y = el.y;
-    a.ybkt = el.ybkt;
+    a.ybkt = el.direct ? el.y : el.ybkt;
+    a.direct = el.direct;
     a.heavy_only = 0;
     a.heavy_separate = 0;
     a.dense_rows = el.dense_rows ? 1 : 0;

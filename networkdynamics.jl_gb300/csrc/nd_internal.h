@@ -132,12 +132,20 @@ constexpr int kWindowIncidences = 2048;  // light window: at most this many inci
 //      in locp, its source block and both lengths come in one 16-byte record per slot.
 // Each edge's function is evaluated once instead of twice, and the edge parameters and
 // the incidence stream are read in order instead of gathered.
+// Where all of y stays in L2 (129 MB) from E to R, the second copy buys nothing: E writes y
+// alone and R gathers from it (`direct`).  Whole RHS, grouped copy against direct, µs: FP32
+// BA(n, 4), n = 1M 61.7 / 57.6, 3M 152 / 142, 6M (96 MB of y) 291 / 285, 8M 385 / 408, 10M
+// 482 / 551; FP64 BA(n, 4), n = 1M 88.4 / 78.1, 3M (96 MB) 205 / 187, 5M 334 / 322, 7M
+// 488 / 494; WS(2e6, 20), FP32 188 / 156; WS(3000, 1500), FP64 102 / 94.
 constexpr int kEdgeChunk = 2048;  // edges per phase-E block
 constexpr int kBuckets = 64;
+constexpr int64_t kDirectMaxBytes = 96ll << 20;  // direct up to this size of y
+constexpr int kDirectChunk = 1024;               // edges per phase-E block there, 4 per thread
 
 struct EdgeLayout {
     bool enabled = false;
-    int64_t n_chunks = 0;
+    bool direct = false;  // no ybkt: locp holds positions of y
+    int64_t n_chunks = 0;  // phase-E blocks
     int32_t* esrc = nullptr;   // [ne]
     int32_t* edst = nullptr;   // [ne]
     uint16_t* lslot = nullptr;     // [ne] slot of edge e in its chunk's (bucket, edge)-ordered staging
@@ -154,7 +162,7 @@ struct EdgeLayout {
     // row phase takes its dense-network kernel
     bool dense_rows = false;
     int32_t n_warp_f32 = 0;  // medium rows of at least kWarpRowMinF32 terms (the first medium slots)
-    void* ybkt = nullptr;      // [ne] scratch
+    void* ybkt = nullptr;      // [ne] scratch (lslot, run_start, run_base and ybkt: NULL when direct)
 };
 
 struct Topology {
@@ -209,6 +217,7 @@ struct RhsArgs {
     const int32_t* locp;
     void* y;
     void* ybkt;
+    bool direct;  // ybkt is y
     int32_t dense_rows;  // the row phase runs dense_row_kernel (see EdgeLayout::dense_rows)
     int32_t n_warp_f32;  // FP32: the first medium slots with >= kWarpRowMinF32 terms, a warp each
 };

@@ -50,3 +50,37 @@ def test_rhs_at_layout_limits(cuda, graph, vk, ek):
     got = gpu_rhs(nd.adapt(net, torch.float32), u32, p32, cuda, np.float32)
     scale = on.abs_terms(u32.astype(np.float64), p32.astype(np.float64)) + np.abs(ref)
     assert np.all(np.abs(got - ref) <= 4e-6 * scale)
+
+
+@pytest.mark.parametrize("ne,dtype", [
+    (2_100_001, np.float64), (2_100_002, np.float64), (2_100_003, np.float64), (2_100_000, np.float32),
+    (2_100_003, np.float32), (2_100_004, np.float32),            # every remainder of four edges per thread
+    (96 * 2**17 - 1, np.float64), (96 * 2**17, np.float64), (96 * 2**17 + 1, np.float64),  # 96 MiB of edge values
+])
+@pytest.mark.parametrize("nv", [300_000, 300_001])  # edge parameters on and off a 16-byte boundary
+def test_two_phase_edge_values(cuda, ne, dtype, nv):
+    """Rows that gather from the edge values or from their grouped copy against the fused layout:
+    the same bits in FP64; FP32 within 4e-6 of the term scale of either (24 eps of a compensated
+    sum), so within twice that of each other."""
+    import torch
+    rng = np.random.default_rng(ne + nv)
+    a, b = rng.integers(0, nv, size=(2, ne + ne // 8))
+    key = np.unique(np.minimum(a, b)[a != b] * np.int64(nv) + np.maximum(a, b)[a != b])
+    assert key.size >= ne
+    key = np.sort(rng.permutation(key)[:ne])
+    src, dst = np.ascontiguousarray(key // nv), np.ascontiguousarray(key % nv)
+    net = nd.adapt(nd.Network(nd.Graph(nv, src, dst), nd.diffusion_vertex(), nd.diffusion_edge()),
+                   torch.float64 if dtype == np.float64 else torch.float32)
+    u, p = rng.normal(size=nv).astype(dtype), rng.uniform(0.5, 1.5, size=ne).astype(dtype)
+    net.set_layout("auto")
+    auto = gpu_rhs(net, u, p, cuda, dtype)
+    # 2.1e6 edges are the last that FP32 takes in one launch
+    assert net.kernel_times()["edge_phase"][0] == (0 if dtype == np.float32 and ne == 2_100_000 else 1)
+    net.set_layout("fused")
+    fused = gpu_rhs(net, u, p, cuda, dtype)
+    if dtype == np.float64:
+        np.testing.assert_array_equal(auto, fused)
+    else:
+        term = np.abs(p.astype(np.float64) * (u[src].astype(np.float64) - u[dst]))
+        scale = np.bincount(src, term, nv) + np.bincount(dst, term, nv)
+        assert np.all(np.abs(auto.astype(np.float64) - fused) <= 8e-6 * scale)
