@@ -189,12 +189,27 @@ __device__ __forceinline__ Cx<T> cmul(Cx<T> a, Cx<T> b) {
     return {A::sub(A::mul(a.r, b.r), A::mul(a.i, b.i)), A::add(A::mul(a.r, b.i), A::mul(a.i, b.r))};
 }
 
+// Comparisons of the complex division on the bits in FP64: a DSETP takes the FP64 pipe as long as
+// an add does.  (A NaN compares as a magnitude above infinity; the quotient is NaN either way.)
+template <typename T>
+__device__ __forceinline__ bool abs_le(T a, T b) {
+    return fabs(a) <= fabs(b);
+}
+__device__ __forceinline__ bool abs_le(double a, double b) {
+    return (__double_as_longlong(a) & INT64_MAX) <= (__double_as_longlong(b) & INT64_MAX);
+}
+template <typename T>
+__device__ __forceinline__ bool nonzero(T a) {
+    return a != T(0);
+}
+__device__ __forceinline__ bool nonzero(double a) { return (__double_as_longlong(a) << 1) != 0; }
+
 template <typename T>
 __device__ __forceinline__ T cdiv_part(T a, T b, T c, T d, T r, T t) {
     using A = Arith<T>;
-    if (r != T(0)) {
+    if (nonzero(r)) {
         const T br = A::mul(b, r);
-        return br != T(0) ? A::mul(A::add(a, br), t) : A::add(A::mul(a, t), A::mul(A::mul(b, t), r));
+        return nonzero(br) ? A::mul(A::add(a, br), t) : A::add(A::mul(a, t), A::mul(A::mul(b, t), r));
     }
     return A::mul(A::add(a, A::mul(d, A::div(b, c))), t);
 }
@@ -203,7 +218,7 @@ template <typename T>
 __device__ __forceinline__ Cx<T> cdiv(Cx<T> x, Cx<T> y) {
     using A = Arith<T>;
     T a = x.r, b = x.i, c = y.r, d = y.i;
-    const bool swap = !(fabs(d) <= fabs(c));
+    const bool swap = !abs_le(d, c);
     if (swap) {
         T t0 = a;
         a = b;
@@ -238,40 +253,57 @@ __device__ __forceinline__ void piline_g(Cx<T> vs, Cx<T> vd, T L, T R, T C1, T C
 }
 
 // Vertex f of the power-grid vertices with the aggregated complex current `in`.
-//   pq!   (benchmark_models.jl:65-73)  algebraic bus: du = S / conj(i), S = P + iQ
+//   pq!   (benchmark_models.jl:65-73)  algebraic bus: du = S / conj(i), S = P + iQ (cdiv)
 //   gen!  (benchmark_models.jl:76-109) 4-state generator (u_r, u_i, θ, ω)
-template <typename T, int VK>
-__device__ __forceinline__ void vertex_f2_at(T* __restrict__ du, const T* __restrict__ u, const T* __restrict__ p,
-                                             int64_t s, int64_t q, Cx<T> in) {
+// The generator's state, parameters and what follows from them alone, so that a caller can have it
+// at hand before the aggregate arrives.
+template <typename T>
+struct Generator {
+    T P, D, E_f, dX_q, dX_d, dX_dash, inv_d, inv_q, Om_H, w, ct, st;
+    Cx<T> uc;
+};
+
+template <typename T>
+__device__ __forceinline__ Generator<T> generator_at(const T* __restrict__ u, const T* __restrict__ p, int64_t s,
+                                                     int64_t q) {
     using A = Arith<T>;
-    if constexpr (VK == ND_V_PQ) {
-        const Cx<T> uc = cdiv<T>({ldv(p + q), ldv(p + q + 1)}, {in.r, -in.i});
-        du[s] = uc.r;
-        du[s + 1] = uc.i;
-    } else {
-        const T H = ldv(p + q), P = ldv(p + q + 1), D = ldv(p + q + 2), Om = ldv(p + q + 3);
-        const T E_f = ldv(p + q + 4), T_d_dash = ldv(p + q + 5), T_q_dash = ldv(p + q + 6);
-        const T X_q_dash = ldv(p + q + 7), X_d_dash = ldv(p + q + 8), X_d = ldv(p + q + 9);
-        const T X_q = ldv(p + q + 10);
-        const T Om_H = A::div(Om, A::mul(T(2), H));
-        const Cx<T> uc = {u[s], u[s + 1]};
-        const T th = u[s + 2], w = u[s + 3];
-        const T ct = A::cos_phase(th), st = A::sin_phase(th);
-        const Cx<T> em = {ct, -st};                        // exp(-im*θ) = (cos θ, -sin θ)
-        const Cx<T> i_c = cmul<T>({-in.i, in.r}, em);     // (im*i)*exp(-im*θ)
-        const Cx<T> e_c = cmul<T>({-uc.i, uc.r}, em);     // (im*u)*exp(-im*θ)
-        const T pw = cmul<T>(uc, {in.r, -in.i}).r;        // real(u*conj(i))
-        const T de_d = A::mul(A::div(T(1), T_q_dash), A::add(-e_c.r, A::mul(A::sub(X_q, X_q_dash), i_c.i)));
-        const T de_q = A::mul(A::div(T(1), T_d_dash),
-                              A::add(A::sub(-e_c.i, A::mul(A::sub(X_d, X_d_dash), i_c.r)), E_f));
-        const Cx<T> t1 = cmul<T>({de_q, -de_d}, {ct, st}); // (-im*de_c)*exp(im*θ)
-        du[s] = A::add(t1.r, A::mul(-uc.i, w));            // + (u*im)*ω
-        du[s + 1] = A::add(t1.i, A::mul(uc.r, w));
-        du[s + 2] = w;
-        du[s + 3] = A::mul(A::sub(A::sub(A::sub(P, A::mul(D, w)), pw),
-                                  A::mul(A::mul(A::sub(X_q_dash, X_d_dash), i_c.r), i_c.i)),
-                           Om_H);
-    }
+    const T H = ldv(p + q), P = ldv(p + q + 1), D = ldv(p + q + 2), Om = ldv(p + q + 3);
+    const T E_f = ldv(p + q + 4), T_d_dash = ldv(p + q + 5), T_q_dash = ldv(p + q + 6);
+    const T X_q_dash = ldv(p + q + 7), X_d_dash = ldv(p + q + 8), X_d = ldv(p + q + 9);
+    const T X_q = ldv(p + q + 10);
+    Generator<T> g;
+    g.uc = {u[s], u[s + 1]};
+    const T th = u[s + 2];
+    g.w = u[s + 3];
+    g.P = P;
+    g.D = D;
+    g.E_f = E_f;
+    g.dX_q = A::sub(X_q, X_q_dash);
+    g.dX_d = A::sub(X_d, X_d_dash);
+    g.dX_dash = A::sub(X_q_dash, X_d_dash);
+    g.inv_d = A::div(T(1), T_d_dash);
+    g.inv_q = A::div(T(1), T_q_dash);
+    g.Om_H = A::div(Om, A::mul(T(2), H));
+    g.ct = A::cos_phase(th);
+    g.st = A::sin_phase(th);
+    return g;
+}
+
+template <typename T>
+__device__ __forceinline__ void generator_f(T* __restrict__ du, int64_t s, const Generator<T>& g, Cx<T> in) {
+    using A = Arith<T>;
+    const Cx<T> em = {g.ct, -g.st};                       // exp(-im*θ) = (cos θ, -sin θ)
+    const Cx<T> i_c = cmul<T>({-in.i, in.r}, em);         // (im*i)*exp(-im*θ)
+    const Cx<T> e_c = cmul<T>({-g.uc.i, g.uc.r}, em);     // (im*u)*exp(-im*θ)
+    const T pw = cmul<T>(g.uc, {in.r, -in.i}).r;          // real(u*conj(i))
+    const T de_d = A::mul(g.inv_q, A::add(-e_c.r, A::mul(g.dX_q, i_c.i)));
+    const T de_q = A::mul(g.inv_d, A::add(A::sub(-e_c.i, A::mul(g.dX_d, i_c.r)), g.E_f));
+    const Cx<T> t1 = cmul<T>({de_q, -de_d}, {g.ct, g.st});  // (-im*de_c)*exp(im*θ)
+    du[s] = A::add(t1.r, A::mul(-g.uc.i, g.w));             // + (u*im)*ω
+    du[s + 1] = A::add(t1.i, A::mul(g.uc.r, g.w));
+    du[s + 2] = g.w;
+    du[s + 3] = A::mul(A::sub(A::sub(A::sub(g.P, A::mul(g.D, g.w)), pw), A::mul(A::mul(g.dX_dash, i_c.r), i_c.i)),
+                       g.Om_H);
 }
 
 }  // namespace nd

@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kJacBlock) jac_powergrid_kernel(JacArgs<T> a) 
         for (int c = 0; c < 4; ++c) uu[c] = D6::seed(__ldg(a.u + s + c), c);
 #pragma unroll
         for (int c = 0; c < 11; ++c) pp[c] = D6(__ldg(a.p + q + c));
-        vertex_f2_at<D6, ND_V_GENERATOR>(out, uu, pp, 0, 0, cx_seed<T, 6>(ir, ii, 4));
+        generator_f<D6>(out, 0, generator_at<D6>(uu, pp, 0, 0), cx_seed<T, 6>(ir, ii, 4));
 #pragma unroll
         for (int f = 0; f < 4; ++f) {
 #pragma unroll

@@ -48,6 +48,7 @@ template <typename T, int VK, int EK>
 __global__ void __launch_bounds__(kBlock) edge_phase_kernel(RhsArgs a) {
     using P2 = typename Pair<T>::type;
     constexpr int DV = VertexDims<VK>::dim;
+    dependents_may_start();
     __shared__ T stage[kEdgeChunk];
     __shared__ uint16_t rstart[kBuckets + 1];
     __shared__ int32_t rbase[kBuckets];
@@ -125,6 +126,7 @@ template <typename T, int VK, int EK>
 __global__ void __launch_bounds__(kBlock) edge_direct_kernel(RhsArgs a) {
     using P2 = typename Pair<T>::type;
     constexpr int DV = VertexDims<VK>::dim;
+    dependents_may_start();
     const T* __restrict__ u = static_cast<const T*>(a.u);
     const T* __restrict__ pe = static_cast<const T*>(a.p) + a.nv * VertexDims<VK>::pdim;
     T* __restrict__ y = static_cast<T*>(a.y);
@@ -182,10 +184,13 @@ __device__ __forceinline__ void warp_row_f32(const RhsArgs& a, int64_t slot) {
     const int4 rm = ld_hint(a.rmeta + slot, stream);
     const int nd = rm.w & 0xffff;
     const int n = nd + (int)((uint32_t)rm.w >> 16);
+    wait_for_primary();
     float acc = 0.f, comp = 0.f;
     for (int j = lane; j < n; j += 32) {
-        const float term = j < nd ? ld_hint(ybkt + ld_hint(a.locp + rm.y + j, stream), stream)
-                                  : -ld_hint(y + (uint32_t)rm.z + (uint32_t)(j - nd), stream);
+        const bool dst = j < nd;
+        const float t = ld_edge(dst ? ybkt + ld_hint(a.locp + rm.y + j, stream) : y + (uint32_t)rm.z + (uint32_t)(j - nd),
+                                stream, true);
+        const float term = dst ? t : -t;
         const float yk = A::sub(term, comp);
         const float s2 = A::add(acc, yk);
         comp = A::sub(A::sub(s2, acc), yk);
@@ -251,9 +256,9 @@ __device__ __forceinline__ void row_thread(const RhsArgs& a, int64_t slot) {
     };
     // The adds of a batch stop at the longest remaining run in the warp (a warp-uniform
     // bound), so a warp issues no add for batch slots that none of its rows has.
-    for (int j0 = 0; j0 < nd; j0 += kBatch) {
-        // the batch's positions as 16-byte vectors (the row's run starts on a multiple of 4)
-        int li[kBatch];
+    // a batch's positions as 16-byte vectors (the row's run starts on a multiple of 4)
+    int li[kBatch];
+    auto load_positions = [&](int j0) {
 #pragma unroll
         for (int k4 = 0; k4 < kBatch / 4; ++k4) {
             const int4 q = j0 + 4 * k4 < nd ? ld_hint(reinterpret_cast<const int4*>(a.locp + lp + j0) + k4, stream)
@@ -263,9 +268,17 @@ __device__ __forceinline__ void row_thread(const RhsArgs& a, int64_t slot) {
             li[4 * k4 + 2] = q.z;
             li[4 * k4 + 3] = q.w;
         }
+    };
+    // FP32 has the registers to hold the first batch's positions over the wait and a batch's over
+    // the adds of the one before; FP64 would spill
+    constexpr bool kAhead = sizeof(T) == 4;
+    if (kAhead) load_positions(0);
+    wait_for_primary();
+    for (int j0 = 0; j0 < nd; j0 += kBatch) {
+        if (!kAhead) load_positions(j0);
         T t[kBatch];
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) t[k] = j0 + k < nd ? ld_hint(ybkt + li[k], ypol) : T(0);
+        for (int k = 0; k < kBatch; ++k) t[k] = ld_edge(ybkt + li[k], ypol, j0 + k < nd);
         const int lim = __reduce_max_sync(__activemask(), (unsigned)min(kBatch, nd - j0));
 #pragma unroll
         for (int k = 0; k < kBatch; ++k) {
@@ -278,6 +291,7 @@ __device__ __forceinline__ void row_thread(const RhsArgs& a, int64_t slot) {
                 add(t[k], false);
             }
         }
+        if (kAhead) load_positions(j0 + kBatch);
     }
     for (int j0 = 0; j0 < ns; j0 += kBatch) {
         // the source block's values as aligned pairs (y has two padding entries at its end;
@@ -289,7 +303,7 @@ __device__ __forceinline__ void row_thread(const RhsArgs& a, int64_t slot) {
         T e[kBatch + 2];
 #pragma unroll
         for (int k2 = 0; k2 < kBatch / 2 + 1; ++k2) {
-            const P2 v = 2 * k2 < avail ? ld_hint(yp + k2, ypol) : P2{T(0), T(0)};
+            const P2 v = ld_edge(yp + k2, ypol, 2 * k2 < avail);
             e[2 * k2] = v.x;
             e[2 * k2 + 1] = v.y;
         }
@@ -413,11 +427,12 @@ __global__ void __launch_bounds__(kDenseBlock) dense_row_kernel(RhsArgs a) {
             }
         };
         load_pos(0);
+        wait_for_primary();
         pipelined_sum<T, KB>(
             nd,
             [&](int j0, T (&t)[KB]) {
 #pragma unroll
-                for (int k = 0; k < KB; ++k) t[k] = j0 + k < nd ? ld_hint(ybkt + pos[k], ypol) : T(0);
+                for (int k = 0; k < KB; ++k) t[k] = ld_edge(ybkt + pos[k], ypol, j0 + k < nd);
                 load_pos(j0 + KB);  // the positions of the batch after
             },
             [&](T t) {  // 0 + t of the first term is the reference's zero start
@@ -430,7 +445,7 @@ __global__ void __launch_bounds__(kDenseBlock) dense_row_kernel(RhsArgs a) {
         ns,
         [&](int j0, T (&t)[KB]) {
 #pragma unroll
-            for (int k = 0; k < KB; ++k) t[k] = j0 + k < ns ? ld_hint(y + sp + (uint32_t)(j0 + k), ypol) : T(0);
+            for (int k = 0; k < KB; ++k) t[k] = ld_edge(y + sp + (uint32_t)(j0 + k), ypol, j0 + k < ns);
         },
         [&](T t) {
             if constexpr (sizeof(T) == 8) acc = __dsub_rn(acc, t);
@@ -449,17 +464,14 @@ cudaError_t launch_typed(const RhsArgs& a, cudaStream_t s, int phases) {
     // rows below the heavy ones; every summation order adds them sequentially
     const int64_t rows = a.nv - a.n_heavy;
     if (!(phases & kPhaseRow) || rows <= 0) return cudaGetLastError();
+    const auto blocks = [](int64_t n, int per) { return (unsigned)((n + per - 1) / per); };
     if (a.dense_rows && sizeof(T) == 4)
-        dense_warp_row_kernel<VK><<<(unsigned)((rows + kWarpsPerBlock - 1) / kWarpsPerBlock), kBlock, 0, s>>>(a);
-    else if (a.dense_rows)
-        dense_row_kernel<T, VK><<<(unsigned)((rows + kDenseBlock - 1) / kDenseBlock), kDenseBlock, 0, s>>>(a);
-    else if (sizeof(T) == 4 && a.n_warp_f32 > 0)
-        row_phase_f32_kernel<VK><<<(unsigned)((a.n_warp_f32 + kWarpsPerBlock - 1) / kWarpsPerBlock +
-                                              (rows - a.n_warp_f32 + kBlock - 1) / kBlock),
-                                   kBlock, 0, s>>>(a);
-    else
-        row_phase_kernel<T, VK><<<(unsigned)((rows + kBlock - 1) / kBlock), kBlock, 0, s>>>(a);
-    return cudaGetLastError();
+        return launch_secondary(dense_warp_row_kernel<VK>, blocks(rows, kWarpsPerBlock), kBlock, s, a);
+    if (a.dense_rows) return launch_secondary(dense_row_kernel<T, VK>, blocks(rows, kDenseBlock), kDenseBlock, s, a);
+    if (sizeof(T) == 4 && a.n_warp_f32 > 0)
+        return launch_secondary(row_phase_f32_kernel<VK>,
+                                blocks(a.n_warp_f32, kWarpsPerBlock) + blocks(rows - a.n_warp_f32, kBlock), kBlock, s, a);
+    return launch_secondary(row_phase_kernel<T, VK>, blocks(rows, kBlock), kBlock, s, a);
 }
 
 template <typename T>

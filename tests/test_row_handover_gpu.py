@@ -1,0 +1,80 @@
+"""The row kernels that start beside the last blocks of their edge kernel: rows of every length
+around their batch of terms, and calls one behind the other, each reading its own edges."""
+import numpy as np
+import pytest
+
+import nd_gb300 as nd
+from oracle import oracle as O
+
+from ndtest import gpu_rhs
+
+pytestmark = pytest.mark.gpu
+
+
+def hub_graph(degrees, nv):
+    k = len(degrees)
+    e = sorted((h, k + i) for h, d in enumerate(degrees) for i in range(d))
+    arr = np.array(e, dtype=np.int64)
+    return nd.Graph(nv, np.ascontiguousarray(arr[:, 0]), np.ascontiguousarray(arr[:, 1]))
+
+
+@pytest.mark.parametrize("nv", [63, 64, 65, 129])  # around the blocks of 64 rows and lines
+def test_powergrid_rows(cuda, nv):
+    """Rows of 0 to 17 lines; lines without resistance, without reactance and without either (both
+    branches of the complex division, its zero numerators, and infinities).  No sine: the
+    oracle's bits."""
+    import torch
+    g = hub_graph([0, 1, 2, 3, 4, 5, 7, 8, 9, 12, 13, 16, 17], nv)
+    net = nd.Network(g, [nd.pqnode()] * nv, nd.piline())
+    on = O.OracleNetwork.from_batches(g.nv, g.src, g.dst, [m.kind for m in net.vertex_batches], net.vertex_batch,
+                                      [(O.E_PILINE, O.C_FIDUCIAL)], net.edge_batch)
+    rng = np.random.default_rng(nv)
+    u, p = rng.normal(size=net.dim), rng.uniform(0.5, 1.5, size=net.pdim)
+    line = p[net.pdim - 4 * g.ne:].reshape(-1, 4)
+    line[0::5, 1] = 0.0
+    line[1::5, 0] = 0.0
+    line[7, :2] = 0.0
+    u[2 * g.dst[3]:2 * g.dst[3] + 2] = u[2 * g.src[3]:2 * g.src[3] + 2]
+    np.testing.assert_array_equal(gpu_rhs(nd.adapt(net, torch.float64), u, p, cuda, np.float64), on.rhs(u, p))
+
+
+@pytest.mark.parametrize("kind", ["powergrid", "mixed", "two-phase", "dense"])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_calls_in_a_row(cuda, kind, dtype):
+    """Twelve calls on twelve states without a synchronisation between them, plain and replayed
+    from a captured graph, have the bits of calls made one at a time."""
+    import torch
+    dt = getattr(torch, dtype)
+    if kind == "powergrid":
+        g = nd.watts_strogatz(3000, 4, 0.5, seed=1)
+        net = nd.Network(g, [nd.pqnode() if i % 3 else nd.generator() for i in range(g.nv)], nd.piline())
+    elif kind == "mixed":
+        g = nd.watts_strogatz(3000, 6, 0.5, seed=2)
+        net = nd.Network(g, [nd.kuramoto_first() if i % 2 else nd.kuramoto_second() for i in range(g.nv)],
+                         nd.kuramoto_edge() if hasattr(nd, "kuramoto_edge") else nd.static_line())
+    elif kind == "two-phase":
+        net = nd.Network(nd.watts_strogatz(220_000, 20, 0.3, seed=3), nd.kuramoto_second(), nd.static_line())
+    else:
+        net = nd.Network(nd.watts_strogatz(2200, 1100, 0.0, seed=4), nd.diffusion_vertex(), nd.diffusion_edge())
+    net = nd.adapt(net, dt)
+    gen = torch.Generator(device=cuda).manual_seed(5)
+    u = torch.randn(12, net.dim, dtype=dt, device=cuda, generator=gen)
+    p = torch.rand(net.pdim, dtype=dt, device=cuda, generator=gen) + 0.5
+    ref, got = torch.empty_like(u), torch.zeros_like(u)
+    for i in range(12):
+        net(ref[i], u[i], p, 0.0)
+        torch.cuda.synchronize()
+    for i in range(12):
+        net(got[i], u[i], p, 0.0)
+    torch.cuda.synchronize()
+    assert torch.equal(got, ref)
+    graph = torch.cuda.CUDAGraph()
+    got.zero_()
+    with torch.cuda.graph(graph):
+        for i in range(12):
+            net(got[i], u[i], p, 0.0)
+    for _ in range(3):
+        got.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, ref)
