@@ -14,8 +14,8 @@
 // sums in edge order.  A row is bound by the latency of its gathers (the neighbour, then its
 // state, direction and line weight), so each thread asks for four terms at a time, and the
 // longest rows start first and are split widest: as two launches with a warp for the longest
-// row, BA(5e5, 2) swing took 126 + 50 µs, now 53; a block from 256 terms on (8 round trips for a
-// warp, one or two for the block).
+// row, BA(5e5, 2) swing took 126 + 50 µs, now 41; a block from 256 terms on (two round
+// trips for a warp, one for the block).
 #include "nd_components.cuh"
 #include "nd_internal.h"
 
@@ -38,7 +38,11 @@ __device__ __forceinline__ void jvp_vertex(int64_t v, T acc, const T* __restrict
     }
 }
 
-constexpr int kJvpBlock = 256;
+// Blocks of 128, eight to an SM (64 registers): a block's slots are free again sooner where its rows
+// differ in length.  BA(n, k) swing, FP64, against blocks of 256 at the 72 registers the kernel
+// takes uncapped, µs: (5e5, 2) 41.0 / 47.4, (2e5, 4) 37.1 / 43.0, (5e3, 2) 20.7 / 22.6; 256 by 4
+// 45.2, 128 by 10 44.6, 64 by 16 41.3 on the first.
+constexpr int kJvpBlock = 128;
 
 // Σ over the terms k, k + step, ... < end of a row, four in flight.
 template <typename T, int VK, int EK>
@@ -73,12 +77,12 @@ __device__ __forceinline__ T jvp_sum(uint32_t k, uint32_t end, uint32_t step, co
 }
 
 template <typename T, int VK, int EK>
-__global__ void __launch_bounds__(kJvpBlock) jvp_kernel(int64_t n_block, int64_t n_long, int64_t nv,
-                                                        const uint32_t* __restrict__ slot_ptr,
-                                                        const int32_t* __restrict__ slot_vertex,
-                                                        const int2* __restrict__ incid, const T* __restrict__ u,
-                                                        const T* __restrict__ p, const T* __restrict__ vv,
-                                                        T* __restrict__ jv) {
+__global__ void __launch_bounds__(kJvpBlock, 8) jvp_kernel(int64_t n_block, int64_t n_long, int64_t nv,
+                                                           const uint32_t* __restrict__ slot_ptr,
+                                                           const int32_t* __restrict__ slot_vertex,
+                                                           const int2* __restrict__ incid, const T* __restrict__ u,
+                                                           const T* __restrict__ p, const T* __restrict__ vv,
+                                                           T* __restrict__ jv) {
     using A = Arith<T>;
     constexpr int DV = VertexDims<VK>::dim;
     constexpr int kWarps = kJvpBlock / 32;
