@@ -35,8 +35,8 @@ __device__ __forceinline__ uint64_t policy_evict_normal() {
 }
 
 // ---- a kernel that starts before the one ahead of it in the stream has ended ---------------
-// The row kernels of the two-launch right-hand sides are launched as programmatic dependents of
-// their edge kernel (launch_secondary): once every edge block has started, row blocks take the
+// Row kernels of the two-launch right-hand sides are launched as programmatic dependents of
+// their edge kernel (launch_secondary), where that is the faster way: once every edge block has started, row blocks take the
 // slots that edge blocks free, load what does not depend on the edges, and wait in
 // wait_for_primary until the edge grid has ended and its writes are visible.  What the edges
 // wrote is read by the volatile, coherent loads below (ld_edge), which stay behind the wait;
