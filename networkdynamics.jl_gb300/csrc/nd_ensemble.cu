@@ -275,7 +275,7 @@ __device__ __forceinline__ int take_instance(const EnsArgs& a, int* sh) {
     return *sh;
 }
 
-// max(|a|, |b|) without the FP64 unit (NaN wins, so that it reaches the error norm)
+// max(|a|, |b|) without the FP64 unit (NaN wins, so that it reaches the error norm or the residual)
 __device__ __forceinline__ double max_abs(double a, double b) {
     const uint64_t x = exact::to_bits(a) & ~exact::kSign, y = exact::to_bits(b) & ~exact::kSign;
     return exact::from_bits(x > y ? x : y);
@@ -483,7 +483,8 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
         int it = 0, cgsum = 0, st = ND_OK;
         double res = 0.0;
         for (;;) {
-            // residual of the full RHS at ω = 0: max |(Pm + Σ)/M|, and G
+            // residual of the full RHS at ω = 0: max |(Pm + Σ)/M|, and G.  A NaN in any row is the
+            // maximum: a state that is not finite is never taken for converged.
             double mx = 0.0;
             for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) {
                 const uint32_t beg = a.row_ptr[s.vbase + v], end = a.row_ptr[s.vbase + v + 1];
@@ -494,15 +495,15 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
                 const double M = pv[3 * v], D = pv[3 * v + 1], Pm = pv[3 * v + 2];
                 const double r = A::mul(A::div(1.0, M), A::add(A::sub(Pm, A::mul(D, 0.0)), acc));
                 G[s.vbase + v] = A::add(Pm, acc);
-                mx = fmax(mx, fabs(r));
+                mx = max_abs(mx, r);
             }
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(kFullMask, mx, off));
+            for (int off = 16; off > 0; off >>= 1) mx = max_abs(mx, __shfl_xor_sync(kFullMask, mx, off));
             __syncthreads();
             if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mx;
             __syncthreads();
             res = 0.0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) res = fmax(res, wmax[w]);
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) res = max_abs(res, wmax[w]);
             __syncthreads();
             if (res <= np.tol) break;
             if (!(res == res)) {
