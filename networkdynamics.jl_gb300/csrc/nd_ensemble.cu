@@ -37,8 +37,15 @@ struct nd_ensemble {
     int32_t* incid_nbr = nullptr; // [2ne] local neighbour index
     int32_t* incid_eid = nullptr; // [2ne] local edge index | src-side bit
     int* counter = nullptr;       // work queue
+    // connected components of the instances that have several (swing ensembles in FP64, else NULL),
+    // the largest first: comp_count[n] (0 for a connected instance), comp_first[n] its first entry
+    // of comp_ptr, whose ranges of comp_vertex hold local vertex indices
+    int32_t* comp_count = nullptr;
+    int64_t* comp_first = nullptr;
+    int64_t* comp_ptr = nullptr;
+    int32_t* comp_vertex = nullptr;
     // scratch for the integrator / Newton
-    double* work = nullptr;  // Tsit5: 8 vectors of dim; Newton: 5 vectors of nv + incidence weights
+    double* work = nullptr;  // Tsit5: 8 vectors of dim; Newton: 6 vectors of nv + incidence weights
     size_t work_bytes = 0;
     int tuned_threads = 0;
 };
@@ -447,13 +454,71 @@ __global__ void __launch_bounds__(kMaxThreads) ens_tsit5_kernel(EnsArgs a, Solve
 // each Newton step solves -J δ = G by CG, preconditioned by the diagonal Σ |w| (hubs of a
 // scale-free network spread the diagonal over two orders of magnitude: 306 iterations a
 // solve without it on BA(2000, 2), 106 with it).  G and every Laplacian image are orthogonal to
-// the uniform phase shift; the shift itself, which the preconditioner lets into the solution, is
-// free and taken out at the end.
+// the constants of every connected component (the uniform phase shifts, which the Jacobian does
+// not see).  What rounding leaves of them in the residual no iteration can reduce, and the
+// preconditioner weighs it up where lines are few: once it is most of what is left the
+// directions run along it without bound.  So each component's mean is taken out of the residual
+// at the start and every kProjectEvery iterations.  The shifts that the preconditioner lets into the
+// solution are free and taken out at the end.  Lines of weight 0 can cut a component into parts that
+// the graph does not show: a solve also ends once its direction is such a shift up to rounding
+// (p · A p is below kFlat of p · D p; on a connected graph of n vertices it is above 1 / n² of it).
+constexpr int kProjectEvery = 32;
+constexpr double kFlat = 0x1p-48;
+
+// The components of one instance: `count` ranges of `vertex`, the largest first; count = 0: connected.
+struct Components {
+    int count;
+    const int64_t* ptr;
+    const int32_t* vertex;
+};
+
+// x minus its mean over each component.  Thread t of the block has written x[t], x[t + blockDim.x],
+// ... before and may read them afterwards.  The largest component is the block's, others of more
+// than 32 vertices a warp's, the rest a thread's each.
+template <int NS>
+__device__ void remove_means(double* __restrict__ x, int64_t n, const Components& c, BlockSums<NS>& red) {
+    double m = 0.0;
+    if (c.count == 0) {
+        for (int64_t v = threadIdx.x; v < n; v += blockDim.x) m += x[v];
+        m = block_sum(m, red) / (double)n;
+        for (int64_t v = threadIdx.x; v < n; v += blockDim.x) x[v] -= m;
+        return;
+    }
+    __syncthreads();
+    for (int64_t j = c.ptr[0] + threadIdx.x; j < c.ptr[1]; j += blockDim.x) m += x[c.vertex[j]];
+    m = block_sum(m, red) / (double)(c.ptr[1] - c.ptr[0]);
+    for (int64_t j = c.ptr[0] + threadIdx.x; j < c.ptr[1]; j += blockDim.x) x[c.vertex[j]] -= m;
+    const int lane = threadIdx.x & 31;
+    for (int k = 1 + (int)(threadIdx.x >> 5); k < c.count; k += (int)(blockDim.x >> 5)) {
+        const int64_t b = c.ptr[k], e = c.ptr[k + 1];
+        if (e - b <= 32) break;  // and every one after it
+        double t = 0.0;
+        for (int64_t j = b + lane; j < e; j += 32) t += x[c.vertex[j]];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(kFullMask, t, off);
+        t /= (double)(e - b);
+        for (int64_t j = b + lane; j < e; j += 32) x[c.vertex[j]] -= t;
+    }
+    for (int k = 1 + (int)threadIdx.x; k < c.count; k += (int)blockDim.x) {
+        const int64_t b = c.ptr[k], e = c.ptr[k + 1];
+        if (e - b > 32) continue;
+        double t = 0.0;
+        for (int64_t j = b; j < e; ++j) t += x[c.vertex[j]];
+        t /= (double)(e - b);
+        for (int64_t j = b; j < e; ++j) x[c.vertex[j]] -= t;
+    }
+    __syncthreads();
+}
+
 struct NewtonParams {
     double tol;
     int max_newton, max_cg;
     int64_t nv, ninc;  // packed vertices, incidences (scratch strides)
     double cg_rtol;
+    const int32_t* comp_count;  // NULL: every instance is connected
+    const int64_t* comp_first;
+    const int64_t* comp_ptr;
+    const int32_t* comp_vertex;
 };
 
 template <int EK>
@@ -480,6 +545,9 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
         double* th = U + s.ubase;  // θ at even, ω at odd positions
         const double* pv = p + s.pbase;
         const double* pe = pv + nvi * 3;
+        Components comps{0, nullptr, nullptr};
+        if (np.comp_count && np.comp_count[i] > 0)
+            comps = {np.comp_count[i], np.comp_ptr + np.comp_first[i], np.comp_vertex};
         int it = 0, cgsum = 0, st = ND_OK;
         double res = 0.0;
         for (;;) {
@@ -514,13 +582,7 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
                 st = ND_ERR_MAXITERS;
                 break;
             }
-            // weights, preconditioner and CG start: X = 0, R = G without its mean.  The right-hand
-            // side is kept orthogonal to the uniform shift (it is, up to rounding): a component
-            // along the null space would make CG grow x without bound along it.
-            double gm = 0.0;
-            for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) gm += G[s.vbase + v];
-            gm = block_sum(gm, red) / (double)nvi;
-            double rs[2] = {0.0, 0.0};  // r · r, r · z
+            // weights, preconditioner and CG start: X = 0, R = G without its means
             for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) {
                 const uint32_t beg = a.row_ptr[s.vbase + v], end = a.row_ptr[s.vbase + v + 1];
                 const double uv = th[2 * v];
@@ -532,11 +594,14 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
                     W[k] = EK == ND_E_KURAMOTO ? A::times_cos(Kk, dth) : Kk;
                     d += fabs(W[k]);
                 }
-                const double di = d > 0.0 ? A::div(1.0, d) : 1.0;
-                const double r = G[s.vbase + v] - gm, z = di * r;
-                Di[s.vbase + v] = di;
+                Di[s.vbase + v] = d > 0.0 ? A::div(1.0, d) : 1.0;
                 X[s.vbase + v] = 0.0;
-                R[s.vbase + v] = r;
+                R[s.vbase + v] = G[s.vbase + v];
+            }
+            remove_means(R + s.vbase, nvi, comps, red);
+            double rs[2] = {0.0, 0.0};  // r · r, r · z
+            for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) {
+                const double r = R[s.vbase + v], z = Di[s.vbase + v] * r;
                 Pd[s.vbase + v] = z;
                 rs[0] += r * r;
                 rs[1] += r * z;
@@ -548,7 +613,8 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
             // below the Newton tolerance
             const double floor2 = (1e-3 * np.tol) * (1e-3 * np.tol);
             int cg = 0;
-            while (cg < np.max_cg && rs[0] > np.cg_rtol * np.cg_rtol * rr0 && rs[0] > floor2) {
+            bool flat = false;  // the same in every thread
+            while (!flat && cg < np.max_cg && rs[0] > np.cg_rtol * np.cg_rtol * rr0 && rs[0] > floor2) {
                 double pq = 0.0;
                 for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) {
                     const uint32_t beg = a.row_ptr[s.vbase + v], end = a.row_ptr[s.vbase + v + 1];
@@ -559,6 +625,7 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
                     pq += pvv * acc;
                 }
                 pq = block_sum(pq, red);
+                if (pq == 0.0) break;  // no step along this direction (the same in every thread)
                 const double alpha = rz / pq;
                 rs[0] = rs[1] = 0.0;
                 for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) {
@@ -567,6 +634,18 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
                     R[s.vbase + v] = r;
                     rs[0] += r * r;
                     rs[1] += r * (Di[s.vbase + v] * r);
+                }
+                if (cg % kProjectEvery == kProjectEvery - 1) {
+                    remove_means(R + s.vbase, nvi, comps, red);
+                    rs[0] = rs[1] = 0.0;
+                    double pdp = 0.0;
+                    for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) {
+                        const double r = R[s.vbase + v], pvv = Pd[s.vbase + v], di = Di[s.vbase + v];
+                        rs[0] += r * r;
+                        rs[1] += r * (di * r);
+                        pdp += A::div(pvv * pvv, di);
+                    }
+                    flat = fabs(pq) <= kFlat * block_sum(pdp, red);
                 }
                 block_sums<2>(rs, red);
                 const double beta = rs[1] / rz;
@@ -578,12 +657,10 @@ __global__ void ens_newton_kernel(EnsArgs a, NewtonParams np, double* __restrict
             }
             cgsum += cg;
             __syncthreads();
-            // Newton update θ += δ with -J δ = G (δ = X, taken with zero mean: the uniform
-            // phase shift is free)
-            double xm = 0.0;
-            for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) xm += X[s.vbase + v];
-            xm = block_sum(xm, red) / (double)nvi;
-            for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) th[2 * v] += X[s.vbase + v] - xm;
+            // Newton update θ += δ with -J δ = G (δ = X, taken with zero means: the phase shifts are
+            // free)
+            remove_means(X + s.vbase, nvi, comps, red);
+            for (int64_t v = threadIdx.x; v < nvi; v += blockDim.x) th[2 * v] += X[s.vbase + v];
             ++it;
             __syncthreads();
         }
@@ -678,6 +755,70 @@ cudaError_t ensure_work(nd_ensemble* e, size_t bytes) {
     return err;
 }
 
+// The connected components of the instances that have several (see nd_ensemble).
+struct ComponentsHost {
+    std::vector<int32_t> count, vertex;
+    std::vector<int64_t> first, ptr;
+    bool any = false;
+};
+
+ComponentsHost find_components(const nd_ensemble_desc* d) {
+    ComponentsHost c;
+    const int64_t n = d->n_instances;
+    c.count.assign(n, 0);
+    c.first.assign(n, 0);
+    std::vector<int32_t> root;      // union-find: a smaller vertex of the component, itself at the smallest
+    std::vector<int32_t> size, at;  // of the component of a root: vertices, next place in `vertex`
+    std::vector<int32_t> roots;
+    for (int64_t i = 0; i < n; ++i) {
+        const int64_t vn = d->v_offset[i + 1] - d->v_offset[i];
+        const int64_t eb = d->e_offset[i], en = d->e_offset[i + 1] - eb;
+        // many ensembles solve one graph over and over
+        if (i > 0 && vn == d->v_offset[i] - d->v_offset[i - 1] && en == eb - d->e_offset[i - 1] &&
+            (en == 0 || (std::memcmp(d->src + eb, d->src + eb - en, en * sizeof(int64_t)) == 0 &&
+                         std::memcmp(d->dst + eb, d->dst + eb - en, en * sizeof(int64_t)) == 0))) {
+            c.count[i] = c.count[i - 1];
+            c.first[i] = c.first[i - 1];
+            continue;
+        }
+        root.resize(vn);
+        std::iota(root.begin(), root.end(), 0);
+        auto find = [&](int32_t v) {
+            while (root[v] != v) v = root[v] = root[root[v]];
+            return v;
+        };
+        int64_t left = vn;
+        for (int64_t e = eb; e < eb + en && left > 1; ++e) {
+            const int32_t a = find((int32_t)d->src[e]), b = find((int32_t)d->dst[e]);
+            if (a == b) continue;
+            root[std::max(a, b)] = std::min(a, b);
+            --left;
+        }
+        if (left == 1) continue;
+        c.any = true;
+        c.count[i] = (int32_t)left;
+        c.first[i] = (int64_t)c.ptr.size();
+        size.assign(vn, 0);
+        for (int64_t v = 0; v < vn; ++v) ++size[root[v] = find((int32_t)v)];
+        roots.clear();
+        for (int64_t v = 0; v < vn; ++v)
+            if (root[v] == v) roots.push_back((int32_t)v);
+        std::stable_sort(roots.begin(), roots.end(), [&](int32_t x, int32_t y) { return size[x] > size[y]; });
+        at.resize(vn);
+        const int64_t base = (int64_t)c.vertex.size();
+        int32_t next = 0;
+        for (int32_t r : roots) {
+            c.ptr.push_back(base + next);
+            at[r] = next;
+            next += size[r];
+        }
+        c.ptr.push_back(base + vn);
+        c.vertex.resize(base + vn);
+        for (int64_t v = 0; v < vn; ++v) c.vertex[base + at[root[v]]++] = (int32_t)v;
+    }
+    return c;
+}
+
 void free_ensemble(nd_ensemble* e) {
     cudaFree(e->v0);
     cudaFree(e->e0);
@@ -686,6 +827,10 @@ void free_ensemble(nd_ensemble* e) {
     cudaFree(e->incid_nbr);
     cudaFree(e->incid_eid);
     cudaFree(e->counter);
+    cudaFree(e->comp_count);
+    cudaFree(e->comp_first);
+    cudaFree(e->comp_ptr);
+    cudaFree(e->comp_vertex);
     cudaFree(e->work);
 }
 
@@ -756,6 +901,8 @@ int nd_ensemble_create(const nd_ensemble_desc* d, int dtype, nd_ensemble** out) 
     e->dim = nv * vertex_dim(d->vertex_kind);
     e->pdim = nv * vertex_pdim(d->vertex_kind) + ne * edge_pdim(d->edge_kind);
     e->max_rows = max_rows;
+    ComponentsHost comps;
+    if (dtype == ND_F64 && d->vertex_kind == ND_V_SWING) comps = find_components(d);
     auto up = [&](void** dp, const void* hp, size_t bytes) -> cudaError_t {
         cudaError_t err = cudaMalloc(dp, std::max<size_t>(bytes, 16));
         if (err == cudaSuccess && bytes) err = cudaMemcpy(*dp, hp, bytes, cudaMemcpyHostToDevice);
@@ -768,6 +915,12 @@ int nd_ensemble_create(const nd_ensemble_desc* d, int dtype, nd_ensemble** out) 
         (err = up((void**)&e->row_ptr, row_ptr.data(), sizeof(uint32_t) * (nv + 1))) != cudaSuccess ||
         (err = up((void**)&e->incid_nbr, nbr.data(), sizeof(int32_t) * nbr.size())) != cudaSuccess ||
         (err = up((void**)&e->incid_eid, eid.data(), sizeof(int32_t) * eid.size())) != cudaSuccess ||
+        (comps.any &&
+         ((err = up((void**)&e->comp_count, comps.count.data(), sizeof(int32_t) * n)) != cudaSuccess ||
+          (err = up((void**)&e->comp_first, comps.first.data(), sizeof(int64_t) * n)) != cudaSuccess ||
+          (err = up((void**)&e->comp_ptr, comps.ptr.data(), sizeof(int64_t) * comps.ptr.size())) != cudaSuccess ||
+          (err = up((void**)&e->comp_vertex, comps.vertex.data(), sizeof(int32_t) * comps.vertex.size())) !=
+              cudaSuccess)) ||
         (err = cudaMalloc(&e->counter, sizeof(int))) != cudaSuccess) {
         free_ensemble(e);
         delete e;
@@ -894,7 +1047,8 @@ int nd_ensemble_fixpoint(nd_ensemble* e, double* u, const double* p, double tol,
     if (err != cudaSuccess) return cuda_fail(err, "workspace");
     cudaStream_t s = (cudaStream_t)stream;
     if ((err = cudaMemsetAsync(e->counter, 0, sizeof(int), s)) != cudaSuccess) return cuda_fail(err, "memset");
-    NewtonParams np{tol, max_newton, max_cg, e->nv, 2 * e->ne, 1e-10};
+    NewtonParams np{tol,           max_newton,    max_cg,      e->nv,        2 * e->ne, 1e-10,
+                    e->comp_count, e->comp_first, e->comp_ptr, e->comp_vertex};
     const EnsArgs a = args_of(e);
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
