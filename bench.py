@@ -278,6 +278,39 @@ def run_reference(args, rank, world):
     print(json.dumps(line), flush=True)
 
 
+def secondary_leg(line, key, leg):
+    """line[key] = leg(), or the error: a secondary leg never costs the headline line."""
+    try:
+        line[key] = leg()
+    except Exception as exc:
+        line[key] = {"error": f"{type(exc).__name__}: {exc}"}
+
+
+def ensemble_leg():
+    """Ensemble solves/s, FP32 vs FP64; raises where a state is not a solution."""
+    from nd_gb300 import benchmarks as NB
+    ens = NB.ensemble(4096)
+    keys = ("synchronised_median", "synchronised_p95", "synchronised_max", "synchronised_within_1e-6",
+            "median_instance", "instances_within_1e-6", "desynchronised_median", "sync_verdict_agreement")
+    return {
+        "metric": "ensemble solves/s FP32 vs FP64 @1e-6", "workload": ens["workload"],
+        "instances": 4096, "sync_fraction_f64": ens["sync_fraction_f64"],
+        "solves_per_s_f32_batched": ens["f32"]["solves_per_s"],
+        "solves_per_s_f32x2_batched": ens["f32x2"]["solves_per_s"],
+        "solves_per_s_f64_batched": ens["f64"]["solves_per_s"],
+        "solves_per_s_plain_f64": ens["plain_f64_per_instance"]["solves_per_s"],
+        "f32_batched_vs_plain_f64": ens["f32_batched_vs_plain_f64"],
+        "f32x2_batched_vs_plain_f64": ens["f32x2_batched_vs_plain_f64"],
+        "f32_batched_vs_f64_batched": ens["f32"]["solves_per_s"] / ens["f64"]["solves_per_s"],
+        "final_state_err_vs_f64": {k: {x: ens[f"{k}_final_state_err_vs_f64"][x] for x in keys}
+                                   for k in ("f32", "f32x2", "f64_1ulp", "f64_f32params")},
+        "note": "f32: FP32 RHS on FP32 parameters; f32x2: double-float RHS (pairs of floats on the FP32 "
+                "pipe) on FP64 parameters; f64_1ulp / f64_f32params: FP64 solves with the parameters "
+                "perturbed by one ulp / rounded to FP32 (the sensitivity floor); state, error norm and "
+                "step control are FP64 in every run",
+        "details": ens}
+
+
 def dense_case_leg(dev, steps=200):
     """The reference's dense diffusion benchmark case (diffusion_static_edge at its largest N,
     WS(3000, 1500): rows of 1500 terms), FP64 and FP32: device time per RHS over back-to-back
@@ -504,10 +537,7 @@ def run_gb300(args, rank, world, local):
         line["e2e"]["result_matches_device"] = bool(ok)
     line["clocks"] = clk.summary()
     if world == 1 and not args.no_dense:
-        try:
-            line["reference_dense_case"] = dense_case_leg(dev)
-        except Exception as exc:  # a secondary leg never costs the headline line
-            line["reference_dense_case"] = {"error": f"{type(exc).__name__}: {exc}"}
+        secondary_leg(line, "reference_dense_case", lambda: dense_case_leg(dev))
     # the second half of the headline metric: ensemble solves/s, FP32 vs FP64, and the
     # learned warm start (single-GPU runs; the instances are independent replicas)
     if world == 1 and not (args.no_ensemble and args.no_warmstart):
@@ -515,30 +545,11 @@ def run_gb300(args, rank, world, local):
         del nw, u, p, du
         torch.cuda.empty_cache()
         if not args.no_ensemble:
-            ens = NB.ensemble(4096)
-            keys = ("synchronised_median", "synchronised_p95", "synchronised_max", "synchronised_within_1e-6",
-                    "median_instance", "instances_within_1e-6", "desynchronised_median", "sync_verdict_agreement")
-            line["ensemble"] = {
-                "metric": "ensemble solves/s FP32 vs FP64 @1e-6", "workload": ens["workload"],
-                "instances": 4096, "sync_fraction_f64": ens["sync_fraction_f64"],
-                "solves_per_s_f32_batched": ens["f32"]["solves_per_s"],
-                "solves_per_s_f32x2_batched": ens["f32x2"]["solves_per_s"],
-                "solves_per_s_f64_batched": ens["f64"]["solves_per_s"],
-                "solves_per_s_plain_f64": ens["plain_f64_per_instance"]["solves_per_s"],
-                "f32_batched_vs_plain_f64": ens["f32_batched_vs_plain_f64"],
-                "f32x2_batched_vs_plain_f64": ens["f32x2_batched_vs_plain_f64"],
-                "f32_batched_vs_f64_batched": ens["f32"]["solves_per_s"] / ens["f64"]["solves_per_s"],
-                "final_state_err_vs_f64": {k: {x: ens[f"{k}_final_state_err_vs_f64"][x] for x in keys}
-                                           for k in ("f32", "f32x2", "f64_1ulp", "f64_f32params")},
-                "note": "f32: FP32 RHS on FP32 parameters; f32x2: double-float RHS (pairs of floats on the FP32 "
-                        "pipe) on FP64 parameters; f64_1ulp / f64_f32params: FP64 solves with the parameters "
-                        "perturbed by one ulp / rounded to FP32 (the sensitivity floor); state, error norm and "
-                        "step control are FP64 in every run",
-                "details": ens}
+            secondary_leg(line, "ensemble", ensemble_leg)
             torch.cuda.empty_cache()
         if not args.no_warmstart:
-            ws = NB.warmstart()
-            line["warm_start"] = {"metric": "Newton iterations to residual 1e-10, cold / warm", **ws}
+            secondary_leg(line, "warm_start", lambda: {
+                "metric": "Newton iterations to residual 1e-10, cold / warm", **NB.warmstart()})
             torch.cuda.empty_cache()
     if rank == 0 and world == 1 and not args.no_cpu:
         res = cpu_baseline(g, u_h, w_h)

@@ -32,6 +32,17 @@ def _log(msg):
     print(f"[{time.perf_counter() - _T0:8.1f} s] {msg}", file=sys.stderr, flush=True)
 
 
+def require_solved(what, u, offset, status):
+    """Raises unless every instance of a packed ensemble state (offset[i]:offset[i + 1] is instance
+    i's) has status OK and is finite: no figure is reported over states that are not solutions."""
+    bad = np.flatnonzero(np.asarray(status) != 0)
+    if bad.size:
+        raise RuntimeError(f"{what}: {bad.size} instances not solved, first {bad[0]} (status {status[bad[0]]})")
+    bad = np.flatnonzero(np.add.reduceat(~np.isfinite(u), np.asarray(offset)[:-1].astype(np.int64)))
+    if bad.size:
+        raise RuntimeError(f"{what}: {bad.size} instances with a state that is not finite, first {bad[0]}")
+
+
 def rhs(nv=10_000_000, m=4, dtype="f64", calls=8, seed=1):
     """A few calls of the diffusion RHS on Barabasi-Albert(nv, m) with the headline
     benchmark's seeded inputs (u ~ N(0, 1), w ~ U(0, 1)): the short program that per-kernel
@@ -159,9 +170,9 @@ def ensemble(n=4096, nv_lo=50, nv_hi=5000, t_end=50.0, reltol=1e-6, abstol=1e-6,
             else:
                 scale[i] *= 0.5
             ps[i] = params(i)
-    u0 = fx.u.clone()
     # one perturbed vertex per instance: Δθ ~ U(-π, π), Δω ~ U(-10, 10)
-    uh = u0.cpu().numpy()
+    uh = fx.u.cpu().numpy()
+    require_solved("steady states", uh, e64.u_offset, status_fx)
     for i, g in enumerate(graphs):
         v = int(rng.integers(0, g.nv))
         s = int(e64.u_offset[i]) + 2 * v
@@ -195,6 +206,7 @@ def ensemble(n=4096, nv_lo=50, nv_hi=5000, t_end=50.0, reltol=1e-6, abstol=1e-6,
         _log(f"{name}: solved in {el:.2f} s")
         finals[name] = r.u.cpu().numpy()
         st = r.status.cpu().numpy()
+        require_solved(f"{name} solve", finals[name], e64.u_offset, st)
         out[name] = {"seconds": el, "solves_per_s": n / el, "threads_per_instance": threads,
                      "steps_mean": float(r.nsteps.double().mean().item()), "ok": int((st == 0).sum())}
     # synchronised / desynchronised verdict per instance: max |ω| at T below 0.1
