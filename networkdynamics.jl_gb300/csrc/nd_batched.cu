@@ -483,14 +483,20 @@ cudaError_t launch_typed(const BatchedNet& b, void* du, const void* u, const voi
     a.y2 = b.y2;
     a.row_vals = b.tstate ? u : b.y2;
     a.mode = mode;
+    // rows beside the last blocks of their edge kernel; without edges the kernel ahead is the
+    // caller's, which may be writing u
+    const auto launch_rows = [&](auto* k, int64_t grid, int block, auto... args) {
+        if (b.ne > 0) return launch_secondary(k, (unsigned)grid, block, s, args...);
+        k<<<(unsigned)grid, block, 0, s>>>(args...);
+        return cudaGetLastError();
+    };
     if (b.depth == 2) {
         if ((phases & kPhaseEdge) && b.ne > 0) {
             const int64_t blocks = std::min<int64_t>((b.ne + kRowBlock - 1) / kRowBlock, int64_t(1) << 20);
             batched_edge_kernel2<T><<<(unsigned)blocks, kRowBlock, 0, s>>>(a);
         }
         if (phases & kPhaseRow)
-            return launch_secondary(batched_row_kernel2<T>, (unsigned)((b.nv + kRowBlock - 1) / kRowBlock), kRowBlock,
-                                    s, a);
+            return launch_rows(batched_row_kernel2<T>, (b.nv + kRowBlock - 1) / kRowBlock, kRowBlock, a);
         return cudaGetLastError();
     }
     if ((phases & kPhaseEdge) && b.ne > 0) {
@@ -512,7 +518,7 @@ cudaError_t launch_typed(const BatchedNet& b, void* du, const void* u, const voi
         } else {
             auto* const rows =
                 b.dense_rows ? batched_row_kernel<T, true, 32, false> : batched_row_kernel<T, false, kRowBlock, false>;
-            return launch_secondary(rows, (unsigned)(wb + tb), nt, s, a, wb);
+            return launch_rows(rows, wb + tb, nt, a, wb);
         }
     }
     return cudaGetLastError();

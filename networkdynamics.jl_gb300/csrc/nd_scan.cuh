@@ -644,7 +644,9 @@ static __device__ __forceinline__ double exact_scan_block(double S, const double
 }
 
 
-// Host side: launch `k` as a programmatic dependent of the kernel before it in stream `s`.
+// Host side: launch `k` as a programmatic dependent of the kernel before it in stream `s`.  That
+// kernel is one of the same call, launched normally: what `k` reads before wait_for_primary was
+// complete before that kernel began.  Behind a kernel that is not ours nothing would promise that.
 template <typename... P>
 inline cudaError_t launch_secondary(void (*k)(P...), unsigned grid, int block, cudaStream_t s, P... args) {
     cudaLaunchAttribute attr{};

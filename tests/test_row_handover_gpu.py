@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import nd_gb300 as nd
+from nd_gb300.solve import solve_tsit5
 from oracle import oracle as O
 
 from ndtest import gpu_rhs
@@ -78,3 +79,33 @@ def test_calls_in_a_row(cuda, kind, dtype):
         graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("vertices", ["generators", "swing and kuramoto"])
+@pytest.mark.parametrize("nv", [1, 64, 65, 5000])
+def test_network_without_edges(cuda, vertices, nv):
+    """Rows of a network without edges come behind whatever wrote their states: calls that each
+    follow the kernel writing theirs have the bits of calls made one at a time, which are the
+    oracle's (sines: 1e-13 of the term scale), and Tsit5 runs through."""
+    import torch
+    g = nd.simple_graph(nv, [])
+    if vertices == "generators":
+        net = nd.Network(g, [nd.generator()] * nv, nd.piline())
+    else:
+        net = nd.Network(g, [nd.kuramoto_second() if i % 2 else nd.kuramoto_first() for i in range(nv)], nd.static_line())
+    on = O.OracleNetwork.from_batches(g.nv, g.src, g.dst, [m.kind for m in net.vertex_batches], net.vertex_batch, [], [])
+    rng = np.random.default_rng(nv)
+    us, p = rng.normal(size=(16, net.dim)), rng.uniform(0.5, 1.5, size=net.pdim)
+    nw = nd.adapt(net, torch.float64)
+    ref = np.stack([gpu_rhs(nw, u, p, cuda, np.float64) for u in us])
+    for u, r in zip(us, ref):
+        e = on.rhs(u, p)
+        assert np.all(np.abs(r - e) <= 1e-13 * (10.0 + np.abs(e)))
+    src, pt = torch.from_numpy(us).to(cuda), torch.from_numpy(p).to(cuda)
+    u, got = torch.full((net.dim,), float("nan"), dtype=torch.float64, device=cuda), torch.empty_like(src)
+    for i in range(16):
+        torch.mul(src[i], 1.0, out=u)
+        nw(got[i], u, pt, 0.0)
+    np.testing.assert_array_equal(got.cpu().numpy(), ref)
+    uT, _ = solve_tsit5(nw, torch.from_numpy(0.1 * us[0]).to(cuda), pt, (0.0, 0.5), reltol=1e-8, abstol=1e-10)
+    assert torch.isfinite(uT).all()
