@@ -760,14 +760,40 @@ EnsArgs args_of(nd_ensemble* e) {
     return a;
 }
 
-// Threads per instance when neither the caller nor the autotuner chose: one to two rows of an
-// average instance per thread, within 64 to 512.  More threads than rows idle; fewer leave the
-// largest instances running alone at the end, because an SM then holds so many blocks that
-// every instance starts at once and nothing is left in the queue to balance: 1024 instances of
-// 50 to 2000 vertices took 160, 97, 60 and 60 ms with 64, 128, 256 and 512 threads.
+// Threads per instance when neither the caller nor the autotuner chose.  At most one to two rows of
+// an average instance per thread; more threads than that idle.  Within this limit an SM does the
+// most with 128, unless
+//   - the largest instances would be running alone at the end, because every instance starts at
+//     once and nothing is left in the queue to balance (less than 5 instances of the largest size
+//     per SM), or
+//   - the instances that run side by side (1536 threads' worth per SM) no longer fit in L2 with
+//     their eight vectors.
+// ms with 128 / 256 / 512 threads, FP64, FP32, double-float: 1024 instances of 50 to 2000 vertices
+// 97 / 61 / 56, 56 / 35 / 34, 110 / 83 / 79; 4096 of 50 to 5000 336 / 274 / 272, 214 / 176 / 177,
+// 383 / 369 / 373; 300 of 500 34 / 28 / 25, 18 / 13 / 12, 44 / 37 / 34; 1500 of 600 98 / 97 / 122,
+// 61 / 59 / 71, 110 / 126 / 161; 1500 of 500 79 / 76 / 96, 47 / 48 / 55, 88 / 98 / 127 (its vectors take
+// 96 MB, which double-float, with the most arithmetic per byte, minds least).  Instances of fewer
+// than 128 rows take 128 too (100 of 128 threads busy: 1500 instances 18.7 ms in FP64 against 23.3
+// with 64, 19.1 against 24.4 in double-float), but for FP32 ensembles of one to two waves of
+// blocks of 128, which blocks of 64 take in one (9.1 against 9.6).
 int default_threads(const nd_ensemble* e) {
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
     const int64_t rows = e->nv / e->n_inst;
-    return rows >= 512 ? 512 : (rows >= 256 ? 256 : (rows >= 128 ? 128 : 64));
+    if (rows < 128) {
+        const int64_t wave = 8 * (int64_t)sms;  // blocks of 128 threads of the FP32 kernel (64 registers)
+        return e->dtype == ND_F32 && e->n_inst > wave && e->n_inst <= 2 * wave ? 64 : 128;
+    }
+    const int most = rows >= 512 ? 512 : (rows >= 256 ? 256 : 128);
+    const bool balanced = e->nv / e->max_rows >= 5 * (int64_t)sms;
+    const int64_t fits = (e->dtype == ND_F32X2 ? 120ll : 90ll) << 20;
+    int threads = 128;
+    while (threads < most) {
+        const int64_t side_by_side = std::min<int64_t>(e->n_inst, (int64_t)sms * (1536 / threads));
+        if (balanced && side_by_side * (e->dim / e->n_inst) * 8 * (int64_t)sizeof(double) <= fits) break;
+        threads *= 2;
+    }
+    return threads;
 }
 
 cudaError_t ensure_work(nd_ensemble* e, size_t bytes) {
