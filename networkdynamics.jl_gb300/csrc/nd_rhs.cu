@@ -207,6 +207,30 @@ __global__ void __launch_bounds__(kBlock, 8) rhs_kernel(RhsArgs a) {
 // serial, and on a crowded SM each of its steps waits for other blocks' instructions.
 constexpr int kHeavySoloSmem = 160 * 1024;
 
+// S + the n terms of `tile` (tile_at layout) by hardware adds, in order: a chain of dependent adds
+// (63 clocks each on an SM without other FP64 work), so the next sixteen terms are read from shared
+// memory while sixteen are added.
+__device__ __forceinline__ double chain_sum(double S, const double* __restrict__ tile, int n) {
+    constexpr int kB = 16;
+    double cur[kB], nxt[kB];
+    const int full = n / kB * kB;
+    if (full > 0) {
+#pragma unroll
+        for (int k = 0; k < kB; ++k) cur[k] = tile[tile_at(k)];
+    }
+    for (int i = 0; i < full; i += kB) {
+        const int j = min(i + kB, full - kB);
+#pragma unroll
+        for (int k = 0; k < kB; ++k) nxt[k] = tile[tile_at(j + k)];
+#pragma unroll
+        for (int k = 0; k < kB; ++k) S = __dadd_rn(S, cur[k]);
+#pragma unroll
+        for (int k = 0; k < kB; ++k) cur[k] = nxt[k];
+    }
+    for (int i = full; i < n; ++i) S = __dadd_rn(S, tile[tile_at(i)]);
+    return S;
+}
+
 // FP64 sequential sum of a heavy row by one block: tiles of kScanTile terms, each added by the
 // block-wide exact scan (or the hardware DADD chain in the native mode).  A thread's incidence
 // data of the next tile are in flight while the current tile is added.
@@ -249,8 +273,7 @@ __device__ __forceinline__ void solo_row_fp64(const RhsArgs& a, int slot, double
         __syncthreads();
         load(base + kScanTile);
         if constexpr (MODE == kModeNative) {
-            if (tid < 32)
-                for (int i = 0; i < n; ++i) S = __dadd_rn(S, tile[tile_at(i)]);
+            if (tid < 32) S = chain_sum(S, tile, n);
         } else {
             S = exact_scan_block(S, tile, n, sh);
         }
