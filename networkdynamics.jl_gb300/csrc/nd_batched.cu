@@ -483,10 +483,13 @@ cudaError_t launch_typed(const BatchedNet& b, void* du, const void* u, const voi
     a.y2 = b.y2;
     a.row_vals = b.tstate ? u : b.y2;
     a.mode = mode;
-    // rows beside the last blocks of their edge kernel; without edges the kernel ahead is the
-    // caller's, which may be writing u
+    // Rows start beside the last blocks of their edge kernel.  Not without edges: the kernel ahead is
+    // then the caller's, which may be writing u.  Nor where long FP64 rows are the bulk: these few
+    // one-warp blocks would go several to the first SMs that fall free, whose one FP64 unit their
+    // chains of adds then share, instead of one to an SM (WS(1000, 500), (1900, 950), (3000, 1500):
+    // 81, 154, 258 µs so, 41, 68, 113 after the edge kernel's end).
     const auto launch_rows = [&](auto* k, int64_t grid, int block, auto... args) {
-        if (b.ne > 0) return launch_secondary(k, (unsigned)grid, block, s, args...);
+        if (b.ne > 0 && !b.dense_rows) return launch_secondary(k, (unsigned)grid, block, s, args...);
         k<<<(unsigned)grid, block, 0, s>>>(args...);
         return cudaGetLastError();
     };
