@@ -120,6 +120,12 @@ __device__ __forceinline__ void block_row(const RhsArgs& a, int slot, unsigned c
 }
 
 // ---- windows: a block per window of rows ----------------------------------------------------
+// Up to this many rows above kLightMaxDeg terms in 32 rows are marked by the warp, one after the
+// other; more by a thread each.  FP32, BA(1e5, 2) diffusion / swing, µs: always by the warp 12.6 / 14.6,
+// up to 12 10.4 / 11.6, up to 4 8.5 / 10.4 (never 8.4 / 10.4); a complete graph of 300, FP64, 17.5
+// by the warp and 18.6 by a thread.
+constexpr int kMarkTogether = 4;
+
 template <typename T, int VK, int EK, int MODE>
 __device__ __forceinline__ void window_block(const RhsArgs& a, int win, unsigned char* smem) {
     using A = Arith<T>;
@@ -147,11 +153,13 @@ __device__ __forceinline__ void window_block(const RhsArgs& a, int win, unsigned
         beg = (int)(__ldg(a.slot_ptr + s) - i0);
         end = (int)(__ldg(a.slot_ptr + s + 1) - i0);
         s_uv[tid] = ld_hint(u + v * DV, keep);
-        if (end - beg <= kLightMaxDeg)
-            for (int j = beg; j < end; ++j) s_owner[j] = (uint8_t)tid;
     }
-    // a long row's incidences are marked by its warp
-    for (unsigned m = __ballot_sync(kFull, end - beg > kLightMaxDeg); m; m &= m - 1) {
+    // where a warp has few long rows it marks their incidences together; many, each its own
+    unsigned shared_rows = __ballot_sync(kFull, end - beg > kLightMaxDeg);
+    if (__popc(shared_rows) > kMarkTogether) shared_rows = 0;
+    if (!((shared_rows >> (tid & 31)) & 1u))
+        for (int j = beg; j < end; ++j) s_owner[j] = (uint8_t)tid;
+    for (unsigned m = shared_rows; m; m &= m - 1) {
         const int l = __ffs(m) - 1, e = __shfl_sync(kFull, end, l);
         for (int j = __shfl_sync(kFull, beg, l) + (tid & 31); j < e; j += 32) s_owner[j] = (uint8_t)((tid & ~31) + l);
     }
