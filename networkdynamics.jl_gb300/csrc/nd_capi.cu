@@ -251,7 +251,9 @@ int build_topology(int64_t nv, int64_t ne, const int64_t* src, const int64_t* ds
     t.max_degree = (int32_t)maxdeg;
     t.n_light = (int32_t)light.size();
     t.n_medium = (int32_t)medium.size();
-    t.n_heavy = (int32_t)heavy.size();
+    t.n_heavy = t.n_apart = (int32_t)heavy.size();
+    if (small && edge_elem == 4)
+        while (t.n_apart > 0 && deg[heavy[t.n_apart - 1]] <= (uint32_t)kFusedHubF32) --t.n_apart;
     t.n_windows = (int32_t)win_ptr.size() - 1;
     t.small = small;
     while (t.n_jvp_block < t.n_heavy + t.n_medium && deg[slot_vertex[t.n_jvp_block]] >= (uint32_t)kJvpBlockMin)
@@ -638,15 +640,14 @@ int nd_rhs(nd_handle* h, int dtype, void* du, int64_t n_du, const void* u, int64
     a.ybkt = el.direct ? el.y : el.ybkt;
     a.direct = el.direct;
     a.heavy_only = 0;
-    a.heavy_separate = 0;
     a.dense_rows = el.dense_rows ? 1 : 0;
     a.n_warp_f32 = el.n_warp_f32;
     const bool edge = el.enabled && h->edge_path;
-    // heavy rows: their own kernel, on the side stream; in FP32 on small networks the first blocks
-    // of the fused launch
-    const bool split = h->topo.n_heavy > 0 && !(h->topo.small && h->dtype == ND_F32);
-    a.heavy_separate = split ? 1 : 0;
-    const int64_t main_rows = (split ? 0 : h->topo.n_heavy) + h->topo.n_windows;
+    // heavy rows: their own kernel, on the side stream; in FP32 on small networks all but the longest
+    // are the first blocks of the fused launch
+    a.n_apart = h->topo.n_apart;
+    const bool split = a.n_apart > 0;
+    const int64_t main_rows = h->topo.n_heavy - a.n_apart + h->topo.n_windows;
     cudaError_t err = cudaSuccess;
     if (split) {
         // Heavy rows run concurrently on the handle's side stream, one per SM, computed

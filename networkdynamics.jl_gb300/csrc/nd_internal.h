@@ -102,8 +102,10 @@ constexpr int kFusedDenseRow = 512;
 // (10 µs for 256), less than the launch on the side stream and the block scan of a row that
 // short (diffusion BA(1e4, 4), rows up to 488 terms: 24.7 µs with all in windows, 16.5 with those
 // above 256 in the heavy kernel).  Longer rows: FP64 as above, FP32 a block each in the same
-// launch, from 129 terms on.
-constexpr int kFusedMaxRow = 256, kFusedMaxRowF32 = 128;
+// launch, from 129 terms on, and above kFusedHubF32 terms in the heavy kernel, whose blocks have the
+// registers to keep more gathers in flight (a star, diffusion / swing, µs in the launch and apart:
+// 10000 vertices 10.4 / 24.8 and 9.4 / 21.8, 1e5 58 / 185 and 43 / 149).
+constexpr int kFusedMaxRow = 256, kFusedMaxRowF32 = 128, kFusedHubF32 = 8192;
 constexpr int64_t fused_window_incidences(int64_t ninc) {
     const int64_t w = ninc / 304;
     return w < 256 ? 256 : (w > 2048 ? 2048 : w);
@@ -173,6 +175,7 @@ struct Topology {
     Incidence* incid = nullptr;      // [2ne] incidences in slot order, each row by edge id (fused path)
     int32_t* win_ptr = nullptr;      // [n_windows+1] first slot of each light window
     int32_t n_light = 0, n_medium = 0, n_heavy = 0, n_windows = 0;
+    int32_t n_apart = 0;             // heavy rows of the heavy kernel (the first ones)
     int32_t n_jvp_block = 0;         // slots of at least kJvpBlockMin terms (the first ones)
     bool small = false;              // fused kernel whatever the edge list (fused_max_incidences)
     EdgeLayout edge;
@@ -205,7 +208,7 @@ struct RhsArgs {
     int32_t vertex_kind, edge_kind;
     int32_t mode;
     int32_t heavy_only;      // launch_rhs: only the heavy rows, one per SM
-    int32_t heavy_separate;  // heavy rows are launched separately (heavy_only), not by this launch
+    int32_t n_apart;         // the first heavy rows, launched separately (heavy_only); the others: fused blocks
     // edge-centric layout (see EdgeLayout)
     int64_t ne, n_chunks;
     const int32_t* esrc;

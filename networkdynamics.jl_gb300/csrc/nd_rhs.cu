@@ -201,10 +201,10 @@ __device__ __forceinline__ void window_block(const RhsArgs& a, int win, unsigned
 template <typename T, int VK, int EK, int MODE>
 __global__ void __launch_bounds__(kBlock, 8) rhs_kernel(RhsArgs a) {
     __shared__ __align__(16) unsigned char smem[Smem<T>::kBytes];
-    const int nh = a.heavy_separate ? 0 : a.n_heavy;
+    const int nh = a.n_heavy - a.n_apart;
     const int b = blockIdx.x;
     if (b < nh) {
-        block_row<T, VK, EK, MODE>(a, b, smem);
+        block_row<T, VK, EK, MODE>(a, a.n_apart + b, smem);
     } else {
         window_block<T, VK, EK, MODE>(a, b - nh, smem);
     }
@@ -318,13 +318,13 @@ cudaError_t launch_heavy_solo(const RhsArgs& a, cudaStream_t s) {
             attr_set = smem;
         }
     }
-    heavy_solo_kernel<T, VK, EK, MODE><<<a.n_heavy, scan ? kScanThreads : kBlock, smem, s>>>(a);
+    heavy_solo_kernel<T, VK, EK, MODE><<<a.n_apart, scan ? kScanThreads : kBlock, smem, s>>>(a);
     return cudaGetLastError();
 }
 
 template <typename T, int VK, int EK>
 cudaError_t launch_heavy_typed(const RhsArgs& a, cudaStream_t s) {
-    if (a.n_heavy == 0) return cudaSuccess;
+    if (a.n_apart == 0) return cudaSuccess;
     if constexpr (sizeof(T) == 4) {
         return launch_heavy_solo<T, VK, EK, kModeTree>(a, s);
     } else {
@@ -339,7 +339,7 @@ cudaError_t launch_heavy_typed(const RhsArgs& a, cudaStream_t s) {
 template <typename T, int VK, int EK>
 cudaError_t launch_typed(const RhsArgs& a, cudaStream_t s) {
     if (a.heavy_only) return launch_heavy_typed<T, VK, EK>(a, s);
-    const int grid = (a.heavy_separate ? 0 : a.n_heavy) + a.n_windows;
+    const int grid = a.n_heavy - a.n_apart + a.n_windows;
     if (grid == 0) return cudaSuccess;
     if constexpr (sizeof(T) == 4) {
         rhs_kernel<T, VK, EK, kModeTree><<<grid, kBlock, 0, s>>>(a);

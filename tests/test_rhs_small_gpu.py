@@ -84,3 +84,19 @@ def test_two_phase_edge_values(cuda, ne, dtype, nv):
         term = np.abs(p.astype(np.float64) * (u[src].astype(np.float64) - u[dst]))
         scale = np.bincount(src, term, nv) + np.bincount(dst, term, nv)
         assert np.all(np.abs(auto.astype(np.float64) - fused) <= 8e-6 * scale)
+
+
+@pytest.mark.parametrize("degrees", [(8192,), (8193,), (20_000, 8193, 8192, 129, 128), (9000, 8500, 8193)])
+@pytest.mark.parametrize("vk,ek", [(O.V_DIFFUSION, O.E_DIFFUSION), (O.V_SWING, O.E_KURAMOTO)])
+def test_f32_hubs_of_small_networks(cuda, degrees, vk, ek):
+    """Rows above 8192 terms in the heavy kernel, shorter ones in the fused launch: every row within
+    4e-6 of the FP64 oracle's term scale (24 eps of a compensated sum), and the heavy kernel
+    runs where such a row is there."""
+    g = hubs(list(degrees), 21_000)
+    on = O.OracleNetwork.from_graph(g, vk, ek)
+    u, p = random_inputs(on, vk, np.random.default_rng(len(degrees)), np.float32)
+    import torch
+    nw = nd.adapt(nd.Network(g, VM[vk](), EM[ek]()), torch.float32)
+    got, ref = gpu_rhs(nw, u, p, cuda, np.float32), on.rhs(u.astype(np.float64), p.astype(np.float64))
+    assert np.all(np.abs(got - ref) <= 4e-6 * (on.abs_terms(u.astype(np.float64), p.astype(np.float64)) + np.abs(ref)))
+    assert nw.kernel_times()["heavy_rows"][0] == int(max(degrees) > 8192)
