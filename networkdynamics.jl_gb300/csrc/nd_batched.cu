@@ -134,9 +134,10 @@ constexpr int kWarpRowMinDegF32 = 2 * kLightMaxDeg + 1;
 // Terms per warp tile in shared memory (FP64 warp rows): 16 per lane.
 constexpr int kWarpTile = 512;
 
-// A term of a row: the edge kernel's output, or (kState) an edge state in u, which no kernel of
-// the call writes.  Through the read-only path the latter took 109 µs against 111 of the whole
-// RHS on WS(3000, 1500) in FP64, 26.4 against 27.7 in FP32.
+// A term of a row: the edge kernel's output, or (kState) a value that no kernel of the call still
+// writes: an edge state in u, or an output of an edge kernel that has ended.  Edge states by the
+// read-only path took 109 µs against 111 of the whole RHS on WS(3000, 1500) in FP64, 26.4 against
+// 27.7 in FP32.
 template <bool kState, typename T>
 __device__ __forceinline__ T ld_term(const T* ptr, uint64_t pol, bool on) {
     if constexpr (kState) return on ? __ldg(ptr) : T(0);
@@ -522,7 +523,7 @@ cudaError_t launch_typed(const BatchedNet& b, void* du, const void* u, const voi
         if (wb + tb <= 0) return cudaGetLastError();
         // rows that read the edge states wait for nothing of the edge phase, but beside its blocks
         // their chains of FP64 adds take longer than after it (WS(3000, 1500): 242 µs against 110)
-        if (b.tstate) {
+        if (b.tstate || b.late_rows) {
             auto* const rows =
                 b.dense_rows ? batched_row_kernel<T, true, 32, true> : batched_row_kernel<T, false, kRowBlock, true>;
             rows<<<(unsigned)(wb + tb), nt, 0, s>>>(a, wb);
@@ -804,6 +805,15 @@ int build_batched(const nd_batched_network_desc* d, int elem, BatchedNet* out) {
         int64_t inc_long = 0, inc_short = 0;
         for (int32_t v : shortr) (deg[v] > (uint32_t)kLightMaxDeg ? inc_long : inc_short) += deg[v];
         bn.dense_rows = elem == 8 && inc_long > inc_short;
+        // FP32 rows of more than 512 terms carrying most of a million edges' terms: launched after the
+        // edge phase, their loads by the read-only path.  Starting early hides 2 µs of launch, but
+        // the coherent loads cost these rows a tenth: mixed vertices on WS(1000, 500) 12.5 µs after /
+        // 10.6 early, (1900, 950) 18.6 / 16.6, (2200, 1100) 18.9 / 20.5, (4000, 2000) 51.8 / 58.6; with rows of
+        // 200 terms, WS(20000, 200), 29.0 / 27.0.
+        int64_t inc_late = 0;
+        for (int32_t v : longr)
+            if (deg[v] > 512) inc_late += deg[v];
+        bn.late_rows = elem == 4 && inc_late > ne && ne >= 1000000;
     }
     // networks of ODE edges only: every term is a state of the caller's u
     std::vector<int32_t> tstate;

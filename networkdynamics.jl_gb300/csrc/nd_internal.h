@@ -290,6 +290,7 @@ struct BatchedNet {
     int32_t max_degree = 0;
     int32_t depth = 1;           // output dimension of vertices and edge sides (2: complex)
     int64_t n_warp_rows = 0;     // slots [0, n_warp_rows): the long rows, a warp per row
+    bool late_rows = false;      // FP32 rows so long that they are launched after the edge phase's end
     bool dense_rows = false;
     int32_t n_warp_f32 = 0;  // medium rows of at least kWarpRowMinF32 terms (the first medium slots)     // FP64 thread rows in deep batches (a dense network)
     int2* eu = nullptr;          // [ne] by edge position: u indices of the src / dst vertex outputs

@@ -81,6 +81,32 @@ def test_calls_in_a_row(cuda, kind, dtype):
     assert torch.equal(got, ref)
 
 
+@pytest.mark.parametrize("n,k", [(2000, 998), (2000, 1000), (1600, 1250)])  # 998,000 edges and from 1e6 on
+def test_f32_long_rows_of_mixed_vertices(cuda, n, k):
+    """FP32 rows of about k terms, started beside the edge phase or after it: within 4e-6 of the FP64
+    oracle's term scale (24 eps of a compensated sum), and twelve calls in a row have the bits of
+    calls made one at a time."""
+    import torch
+    g = nd.watts_strogatz(n, k, 0.3, seed=7)
+    net = nd.Network(g, [nd.kuramoto_first() if i % 2 else nd.kuramoto_second() for i in range(n)], nd.kuramoto_edge())
+    on = O.OracleNetwork.from_batches(g.nv, g.src, g.dst, [m.kind for m in net.vertex_batches], net.vertex_batch,
+                                      [(O.E_KURAMOTO, O.C_ANTISYMMETRIC)], net.edge_batch)
+    rng = np.random.default_rng(k)
+    us = rng.normal(size=(12, net.dim)).astype(np.float32)
+    p = rng.uniform(0.5, 1.5, size=net.pdim).astype(np.float32)
+    nw = nd.adapt(net, torch.float32)
+    ref = np.stack([gpu_rhs(nw, u, p, cuda, np.float32) for u in us])
+    for u, r in zip(us[:2], ref):
+        e = on.rhs(u.astype(np.float64), p.astype(np.float64))
+        # |terms| <= K <= 1.5 each; the swing rows' division by M >= 0.5
+        assert np.all(np.abs(r - e) <= 4e-6 * 2.0 * (1.5 * g.degree().max() + 5.0))
+    src, pt = torch.from_numpy(us).to(cuda), torch.from_numpy(p).to(cuda)
+    got = torch.empty_like(src)
+    for i in range(12):
+        nw(got[i], src[i], pt, 0.0)
+    np.testing.assert_array_equal(got.cpu().numpy(), ref)
+
+
 @pytest.mark.parametrize("vertices", ["generators", "swing and kuramoto"])
 @pytest.mark.parametrize("nv", [1, 64, 65, 5000])
 def test_network_without_edges(cuda, vertices, nv):
