@@ -446,10 +446,12 @@ def jacobian(nw: Network, u, p, t=0.0, stream=None):
     import torch
     # the pattern is the network's: its index tensors go to the device once, and every call
     # hands out copies of its own
-    index = nw._jac_index
-    if index is None or index[0].device != u.device:
+    if nw._jac_index is None or nw._jac_index[0].device != u.device:
         rowptr, colidx = jacobian_pattern(nw)
-        index = nw._jac_index = tuple(torch.from_numpy(x.astype(np.int64)).to(u.device) for x in (rowptr, colidx))
+        nw._jac_index = tuple(torch.from_numpy(x.astype(np.int64)).to(u.device) for x in (rowptr, colidx))
+    index = nw._jac_index
+    if stream is not None and not isinstance(stream, torch.cuda.Stream):
+        stream = torch.cuda.ExternalStream(stream.cuda_stream, device=u.device)
     # every tensor of the result belongs to the stream that fills it
     with contextlib.nullcontext() if stream is None else torch.cuda.stream(stream):
         crow, col = (x.clone() for x in index)

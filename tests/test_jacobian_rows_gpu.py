@@ -52,3 +52,19 @@ def test_jvp_rows(cuda, leaves, dtype, tol):
     J = nd.jacobian(nw, u, p).to_dense().double()
     scale = J.abs() @ v.double().abs()
     assert torch.all((J @ v.double() - jv.double()).abs() <= tol * (scale + 1e-300)).item()
+
+
+def test_stream_given_by_its_handle(cuda):
+    """Any object with a cuda_stream attribute names the stream, as for the other calls."""
+    import types
+
+    import torch
+    net = nd.Network(nd.watts_strogatz(50, 4, 0.2, seed=1), nd.kuramoto_first(), nd.kuramoto_edge())
+    nw = nd.adapt(net, torch.float64)
+    u = torch.randn(net.dim, dtype=torch.float64, device=cuda)
+    p = torch.rand(net.pdim, dtype=torch.float64, device=cuda)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    J = nd.jacobian(nw, u, p, stream=types.SimpleNamespace(cuda_stream=side.cuda_stream))
+    torch.cuda.synchronize()
+    assert torch.equal(J.to_dense(), nd.jacobian(nw, u, p).to_dense())
