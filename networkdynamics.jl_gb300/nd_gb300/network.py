@@ -234,7 +234,7 @@ class Network:
         self._layout()
         self._handle = None
         self._dtype = None
-        self._jac_index = None  # (crow, col) of the Jacobian on the device, see jacobian()
+        self._jac_index = None  # ((crow, col) of the Jacobian on the device, their stream), see jacobian()
         if dtype is not None:
             self._create(dtype)
 
@@ -446,14 +446,18 @@ def jacobian(nw: Network, u, p, t=0.0, stream=None):
     import torch
     # the pattern is the network's: its index tensors go to the device once, and every call
     # hands out copies of its own
-    if nw._jac_index is None or nw._jac_index[0].device != u.device:
+    if nw._jac_index is None or nw._jac_index[0][0].device != u.device:
         rowptr, colidx = jacobian_pattern(nw)
-        nw._jac_index = tuple(torch.from_numpy(x.astype(np.int64)).to(u.device) for x in (rowptr, colidx))
-    index = nw._jac_index
+        nw._jac_index = (tuple(torch.from_numpy(x.astype(np.int64)).to(u.device) for x in (rowptr, colidx)),
+                         _raw_stream(None))
+    index, home = nw._jac_index
     if stream is not None and not isinstance(stream, torch.cuda.Stream):
         stream = torch.cuda.ExternalStream(stream.cuda_stream, device=u.device)
     # every tensor of the result belongs to the stream that fills it
     with contextlib.nullcontext() if stream is None else torch.cuda.stream(stream):
+        if _raw_stream(None) != home:  # the copies below may outlive the network
+            for x in index:
+                x.record_stream(torch.cuda.current_stream())
         crow, col = (x.clone() for x in index)
         values = torch.empty(col.numel(), dtype=u.dtype, device=u.device)
     pp = p.data_ptr() if p is not None and p.numel() else None

@@ -54,6 +54,30 @@ def test_jvp_rows(cuda, leaves, dtype, tol):
     assert torch.all((J @ v.double() - jv.double()).abs() <= tol * (scale + 1e-300)).item()
 
 
+def test_index_tensors_outlive_the_network(cuda):
+    """A Jacobian asked for on a busy stream, whose network goes away before the stream gets to it: its
+    index tensors are the pattern, although the memory of the network's own is free by then."""
+    import torch
+    g = nd.barabasi_albert(20_000, 2, seed=4)
+    net = nd.Network(g, nd.kuramoto_second(), nd.static_line())
+    u = torch.randn(net.dim, dtype=torch.float64, device=cuda)
+    p = torch.rand(net.pdim, dtype=torch.float64, device=cuda) + 0.5
+    nw = nd.adapt(net, torch.float64)
+    ref = nd.jacobian(nw, u, p)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(100_000_000)  # some 50 ms
+    J = nd.jacobian(nw, u, p, stream=side)
+    kept = [x.numel() for x in nw._jac_index[0]]
+    nw._jac_index = None
+    trash = [torch.full((n,), -1, dtype=torch.int64, device=cuda) for n in kept for _ in range(4)]
+    torch.cuda.synchronize()
+    assert trash[0][0].item() == -1
+    assert torch.equal(J.crow_indices(), ref.crow_indices()) and torch.equal(J.col_indices(), ref.col_indices())
+    assert torch.equal(J.values(), ref.values())
+
+
 def test_stream_given_by_its_handle(cuda):
     """Any object with a cuda_stream attribute names the stream, as for the other calls."""
     import types
