@@ -245,7 +245,8 @@ int nd_kernel_times(nd_handle* h, int64_t* launches, double* ms, int n);
  *   n_p         must equal info.pdim when pdim > 0, else ND_ERR_ARG (src/coreloop.jl:5-7);
  *               p may be NULL when pdim == 0
  *   t           unused by the library components, may be NaN
- * du, u, p are device pointers in the reference's flat order (no permutation). */
+ * du, u, p are device pointers in the reference's flat order (no permutation).  du may overlap u;
+ * such a call works on a copy of u (a stream-ordered allocation). */
 int nd_rhs(nd_handle* h, int dtype, void* du, int64_t n_du, const void* u, int64_t n_u,
            const void* p, int64_t n_p, double t, void* stream);
 

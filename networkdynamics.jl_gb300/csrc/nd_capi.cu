@@ -588,6 +588,20 @@ int nd_rhs(nd_handle* h, int dtype, void* du, int64_t n_du, const void* u, int64
     }
     if (!du || !u || (h->pdim > 0 && !p)) return fail(ND_ERR_ARG, "nd_rhs: NULL buffer");
     cudaStream_t s = (cudaStream_t)stream;
+    // du over u: rows read their neighbours' states from u, or their edges', while others write du,
+    // so such a call works on a copy of u
+    const size_t bytes = (size_t)h->dim * (h->dtype == ND_F64 ? 8 : 4);
+    const uintptr_t d0 = reinterpret_cast<uintptr_t>(du), u0 = reinterpret_cast<uintptr_t>(u);
+    if (d0 < u0 + bytes && u0 < d0 + bytes) {
+        void* copy = nullptr;
+        cudaError_t err = cudaMallocAsync(&copy, bytes, s);
+        if (err != cudaSuccess) return cuda_fail(err, "nd_rhs: copy of u");
+        err = cudaMemcpyAsync(copy, u, bytes, cudaMemcpyDeviceToDevice, s);
+        const int rc = err == cudaSuccess ? nd_rhs(h, dtype, du, n_du, copy, n_u, p, n_p, t, stream)
+                                          : cuda_fail(err, "nd_rhs: copy of u");
+        err = cudaFreeAsync(copy, s);
+        return rc != ND_OK || err == cudaSuccess ? rc : cuda_fail(err, "nd_rhs: copy of u");
+    }
     if (h->batched.enabled) {
         const BatchedNet& b = h->batched;
         cudaError_t err = cudaSuccess;
