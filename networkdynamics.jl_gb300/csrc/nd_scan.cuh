@@ -439,7 +439,9 @@ struct BlockScanShared {
     int8_t ev_shift[kScanTile];
 };
 
-// The upper word of |m|, one too small for negative m whose lower word is not zero.
+// The upper word of |m|, one too small for negative m whose lower word is zero.  So an exact negative
+// power of two counts to the binade below its own: a sum that is one is refused (its bits there are
+// all ones), and a start that is one only makes the first step an event.
 __device__ __forceinline__ uint32_t abs_hi(int64_t m) {
     const int32_t h = (int32_t)(m >> 32);
     return (uint32_t)(h ^ (h >> 31));

@@ -130,3 +130,94 @@ def test_device_exact_scan_equals_sequential_sum(cuda):
     got = out.cpu().numpy()
     ref = np.array([sequential(s, t) for s, t in zip(s0, segs)])
     assert_bitwise(ref, got)
+
+
+def block_scan(cuda, segs, s0):
+    """The sums of the segments by the block-wide scan: the self-test runs it on every segment number
+    w with w % 8 == 4, so empty segments fill the others."""
+    import torch
+
+    from nd_gb300 import _capi as capi
+    n = 8 * len(segs)
+    length = np.zeros(n, dtype=np.int64)
+    start = np.zeros(n)
+    length[4::8], start[4::8] = [len(s) for s in segs], s0
+    seg = np.concatenate([[0], np.cumsum(length)])
+    d = [torch.from_numpy(x).to(cuda) for x in (np.concatenate(segs), seg, start)]
+    out = torch.empty(n, dtype=torch.float64, device=cuda)
+    capi.check(capi.load().nd_selftest_exact_scan(d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), out.data_ptr(), n,
+                                                  None))
+    return out.cpu().numpy()[4::8]
+
+
+def check_block_scan(cuda, segs, s0):
+    segs = [np.asarray(s, dtype=np.float64) for s in segs]
+    with np.errstate(all="ignore"):
+        ref = np.array([sequential(np.float64(s), t) for s, t in zip(s0, segs)])
+    assert_bitwise(ref, block_scan(cuda, segs, np.asarray(s0, dtype=np.float64)))
+
+
+@pytest.mark.gpu
+def test_block_scan_lengths(cuda):
+    """Every remainder of a thread's four terms, and the ends of a warp's and a tile's share."""
+    rng = np.random.default_rng(1)
+    segs = [rng.uniform(0, 1, n) * (rng.normal(size=n) - 0.3)
+            for n in [1, 2, 3, 4, 5, 127, 128, 129, 511, 512, 513, 514, 515, 516, 1023, 1024, 1025, 3000]]
+    check_block_scan(cuda, segs, np.zeros(len(segs)))
+
+
+@pytest.mark.gpu
+def test_block_scan_across_the_frame(cuda):
+    """Sums that leave the eight binades of the scan's frame at either end, slowly and at once, and come
+    back; mixed signs that keep the sum near zero; terms ten and more binades above it."""
+    rng = np.random.default_rng(2)
+    segs, s0 = [], []
+    for k in range(24):
+        n = int(rng.integers(200, 1500))
+        up = np.exp2(np.linspace(0, 40, n)) * rng.uniform(0.5, 1, n)                      # grows through 40 binades
+        swing = np.cos(np.arange(n) * rng.uniform(0.01, 1.0)) * rng.uniform(0.9, 1.1, n)  # changes sign throughout
+        spikes = rng.normal(size=n) * np.where(rng.random(n) < 0.02, 2.0 ** rng.integers(8, 14, n), 1.0)
+        cancel = rng.normal(size=n)
+        cancel[1::2] = -cancel[::2][:cancel[1::2].size] * (1 + 2.0 ** -rng.integers(20, 52))
+        segs += [up, -up[::-1], swing, spikes, cancel]
+        s0 += [0.0, float(up.sum()), 2.0 ** -30, -1.0, 3.0]
+    check_block_scan(cuda, segs, s0)
+
+
+@pytest.mark.gpu
+def test_block_scan_negative_powers_of_two_and_ties(cuda):
+    """Starts and running sums that are exact powers of two of either sign, reached from both sides, and
+    terms of half an ulp of the binade above and below."""
+    rng = np.random.default_rng(3)
+    segs, s0 = [], []
+    for sign in (-1.0, 1.0):
+        for e in (-1, 0, 1, 7):
+            b = sign * 2.0 ** e
+            ulp = np.spacing(abs(b))
+            for step in (ulp / 4, ulp / 2, ulp, 3 * ulp / 2, 2.0 ** -20 * abs(b)):
+                t = step * rng.integers(-3, 4, 600)
+                segs += [t, np.concatenate([[b / 2, b / 2], t]), np.concatenate([[2 * b, -b], t, [-b, b, -b / 2, -b / 2, b]])]
+                s0 += [b, 0.0, 0.0]
+            # whole numbers: every sum exact, many of them powers of two
+            segs.append(b * rng.integers(-2, 3, 700))
+            s0.append(b)
+    check_block_scan(cuda, segs, s0)
+
+
+@pytest.mark.gpu
+def test_block_scan_special_values(cuda):
+    """Infinities, NaN, overflow, subnormals, signed zeros and zeros only, at both ends and in between."""
+    rng = np.random.default_rng(4)
+    segs, s0 = [], []
+    for bad in (np.inf, -np.inf, np.nan, 1.7e308, -1.7e308, 5e-324, -5e-324, 2.2250738585072014e-308, 0.0, -0.0):
+        for at in (0, 1, 255, 511, 512, 700):
+            t = rng.normal(size=701)
+            t[at] = bad
+            segs += [t, np.full(701, bad)]
+            s0 += [0.0, 0.0]
+    segs += [np.array([np.inf, -np.inf]), np.array([1e308, 1e308, -np.inf]), np.zeros(600), -np.zeros(600),
+             rng.integers(-50, 50, 600) * 5e-324, np.full(600, 1e308), np.concatenate([np.full(300, 1e300), -np.full(300, 1e300)])]
+    s0 += [0.0, 0.0, -0.0, -0.0, 0.0, 0.0, 1.0]
+    segs += [rng.normal(size=300) * 2.0 ** e for e in (-1070, -1040, -1010, 990, 1015)]
+    s0 += [0.0] * 5
+    check_block_scan(cuda, segs, s0)
