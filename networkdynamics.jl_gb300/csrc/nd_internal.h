@@ -207,7 +207,7 @@ struct RhsArgs {
     int32_t n_light, n_medium, n_heavy, n_windows;
     int32_t vertex_kind, edge_kind;
     int32_t mode;
-    int32_t heavy_only;      // launch_rhs: only the heavy rows, one per SM
+    int32_t heavy_only;      // launch_rhs: only the first n_apart heavy rows, in their own kernel
     int32_t n_apart;         // the first heavy rows, launched separately (heavy_only); the others: fused blocks
     // edge-centric layout (see EdgeLayout)
     int64_t ne, n_chunks;
@@ -291,8 +291,7 @@ struct BatchedNet {
     int32_t depth = 1;           // output dimension of vertices and edge sides (2: complex)
     int64_t n_warp_rows = 0;     // slots [0, n_warp_rows): the long rows, a warp per row
     bool late_rows = false;      // FP32 rows so long that they are launched after the edge phase's end
-    bool dense_rows = false;
-    int32_t n_warp_f32 = 0;  // medium rows of at least kWarpRowMinF32 terms (the first medium slots)     // FP64 thread rows in deep batches (a dense network)
+    bool dense_rows = false;     // FP64 thread rows in deep batches (a dense network)
     int2* eu = nullptr;          // [ne] by edge position: u indices of the src / dst vertex outputs
     uint32_t* tptr = nullptr;    // [nv+1] by slot: range of the slot's terms in tidx
     int32_t* tidx = nullptr;     // [2ne] y2 indices of every row's terms, ascending

@@ -8,13 +8,13 @@
 // written once.  There are no output, gather or aggregation buffers.
 //
 // One launch, two roles chosen per block (degree buckets and slot order: nd_internal.h):
-//   heavy   a block per row: the terms of kTile incidences at a time go to shared memory
-//           and warp 0 adds them in order with the exact scan (FP64), or the block sums
-//           thread-strided slices in a fixed tree (FP32 with Kahan, FP64 tree mode);
+//   heavy   (FP32) a block per row, which sums thread-strided slices with Kahan compensation and
+//           joins them in a fixed tree;
 //   window  a block per window of rows: phase A evaluates the window's edge terms, one
 //           incidence per thread (coalesced incidence loads, independent gathers and FP64
 //           operations in flight) into shared memory; phase B sums one row per thread.
-// Heavy blocks come first so the long rows start early.
+// Heavy blocks come first so the long rows start early.  FP64 heavy rows, and the longest FP32
+// ones, have a kernel of their own (heavy_solo_kernel) beside this one.
 //
 // Cache policy: u is gathered at random and is re-read by every incidence, so its loads
 // ask L2 to keep the lines (evict_last); the incidence stream and the edge parameters are
@@ -23,12 +23,8 @@
 // FP64 on GB300 retires ~2 lanes/clock/SM and a DADD holds its sub-partition's FP64 pipe
 // for a full warp even with one lane active.  Window rows (at most kMediumMaxDeg long)
 // add with hardware DADDs, all lanes busy on rows of similar length.  A hub's sum would
-// be a chain of thousands of DADDs on one sub-partition, so it runs on the integer pipes:
-//   * the heavy rows' warp sums use an exact scan: while the running sum S stays inside one binade,
-//     RN(S + t) = S + RN(t / ulp(S)) ulp(S), so a run of additions becomes an integer
-//     prefix sum of the terms scaled to S's ulp.  A lane whose prefix leaves the binade
-//     (or whose scaled term is a tie) ends the run; that one step is done with the exact
-//     adder and the scan resumes.  The result equals the sequential sum bit for bit.
+// be a chain of thousands of DADDs on one sub-partition, so it runs on the integer pipes, by the
+// block-wide exact scan (nd_scan.cuh), whose result equals the sequential sum bit for bit.
 
 #include "nd_components.cuh"
 #include "nd_exact.cuh"
@@ -41,16 +37,14 @@ namespace {
 
 using namespace dev;
 
-// Shared memory of one block, sized for the largest role (light windows in FP64).
+// Shared memory of one block: a window's (a row's block needs a few words of it).
 template <typename T>
 struct Smem {
-    static constexpr int kWin = (kWindowIncidences + kWindow) * (int)sizeof(T) + kWindowIncidences;
-    static constexpr int kHeavy = kTile * (int)sizeof(double);
-    static constexpr int kBytes = kWin > kHeavy ? kWin : kHeavy;
+    static constexpr int kBytes = (kWindowIncidences + kWindow) * (int)sizeof(T) + kWindowIncidences;
 };
 
-// ---- heavy: a block per row ---------------------------------------------------------------
-template <typename T, int VK, int EK, int MODE>
+// ---- heavy: a block per row (FP32, and FP64 in the tree mode) ------------------------------
+template <typename T, int VK, int EK>
 __device__ __forceinline__ void block_row(const RhsArgs& a, int slot, unsigned char* smem) {
     using A = Arith<T>;
     constexpr int DV = VertexDims<VK>::dim;
@@ -63,59 +57,33 @@ __device__ __forceinline__ void block_row(const RhsArgs& a, int slot, unsigned c
     const uint32_t beg = __ldg(a.slot_ptr + slot), end = __ldg(a.slot_ptr + slot + 1);
     const T uv = __ldg(u + v * DV);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if constexpr (sizeof(T) == 8 && MODE != kModeTree) {
-        double* tile = reinterpret_cast<double*>(smem);
-        double S = 0.0;
-        for (uint32_t base = beg; base < end; base += kTile) {
-            const int n = (int)min((uint32_t)kTile, end - base);
+    T* red = reinterpret_cast<T*>(smem);
+    T acc = T(0), comp = T(0);
 #pragma unroll 4
-            for (int i = tid; i < n; i += kBlock) {
-                const int2 inc = ld_hint(incid + base + i, stream);
-                const T un = ld_hint(u + (int64_t)inc.x * DV, keep);
-                const T w = edge_param<T, EK>(pe, inc.y & 0x7fffffff, stream);
-                tile[i] = incidence_term_w<T, EK>(uv, un, w, inc.y < 0);
-            }
-            __syncthreads();
-            if (warp == 0) {
-                if constexpr (MODE == kModeNative) {
-                    if (lane == 0)
-                        for (int i = 0; i < n; ++i) S = __dadd_rn(S, tile[i]);
-                } else {
-                    S = exact_scan_wide(S, tile, n, lane);
-                }
-            }
-            __syncthreads();
+    for (uint32_t k = beg + tid; k < end; k += kBlock) {
+        const int2 inc = ld_hint(incid + k, stream);
+        const T un = ld_hint(u + (int64_t)inc.x * DV, keep);
+        const T w = edge_param<T, EK>(pe, inc.y & 0x7fffffff, stream);
+        const T term = incidence_term_w<T, EK>(uv, un, w, inc.y < 0);
+        if constexpr (sizeof(T) == 4) {
+            const T y = A::sub(term, comp);
+            const T s = A::add(acc, y);
+            comp = A::sub(A::sub(s, acc), y);
+            acc = s;
+        } else {
+            acc = A::add(acc, term);
         }
-        if (tid == 0) vertex_f<T, VK>(static_cast<T*>(a.du), u, p, v, (T)S);
-    } else {
-        T* red = reinterpret_cast<T*>(smem);
-        T acc = T(0), comp = T(0);
-#pragma unroll 4
-        for (uint32_t k = beg + tid; k < end; k += kBlock) {
-            const int2 inc = ld_hint(incid + k, stream);
-            const T un = ld_hint(u + (int64_t)inc.x * DV, keep);
-            const T w = edge_param<T, EK>(pe, inc.y & 0x7fffffff, stream);
-            const T term = incidence_term_w<T, EK>(uv, un, w, inc.y < 0);
-            if constexpr (sizeof(T) == 4) {
-                const T y = A::sub(term, comp);
-                const T s = A::add(acc, y);
-                comp = A::sub(A::sub(s, acc), y);
-                acc = s;
-            } else {
-                acc = A::add(acc, term);
-            }
-        }
-        if constexpr (sizeof(T) == 4) acc = A::sub(acc, comp);
+    }
+    if constexpr (sizeof(T) == 4) acc = A::sub(acc, comp);
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) acc = A::add(acc, __shfl_xor_sync(kFull, acc, off));
-        if (lane == 0) red[warp] = acc;
-        __syncthreads();
-        if (tid == 0) {
-            T s = red[0];
+    for (int off = 16; off > 0; off >>= 1) acc = A::add(acc, __shfl_xor_sync(kFull, acc, off));
+    if (lane == 0) red[warp] = acc;
+    __syncthreads();
+    if (tid == 0) {
+        T s = red[0];
 #pragma unroll
-            for (int w = 1; w < kWarpsPerBlock; ++w) s = A::add(s, red[w]);
-            vertex_f<T, VK>(static_cast<T*>(a.du), u, p, v, s);
-        }
+        for (int w = 1; w < kWarpsPerBlock; ++w) s = A::add(s, red[w]);
+        vertex_f<T, VK>(static_cast<T*>(a.du), u, p, v, s);
     }
 }
 
@@ -126,7 +94,7 @@ __device__ __forceinline__ void block_row(const RhsArgs& a, int slot, unsigned c
 // by the warp and 18.6 by a thread.
 constexpr int kMarkTogether = 4;
 
-template <typename T, int VK, int EK, int MODE>
+template <typename T, int VK, int EK>
 __device__ __forceinline__ void window_block(const RhsArgs& a, int win, unsigned char* smem) {
     using A = Arith<T>;
     constexpr int DV = VertexDims<VK>::dim;
@@ -198,15 +166,16 @@ __device__ __forceinline__ void window_block(const RhsArgs& a, int win, unsigned
     vertex_f<T, VK>(static_cast<T*>(a.du), u, p, v, acc);
 }
 
-template <typename T, int VK, int EK, int MODE>
+template <typename T, int VK, int EK>
 __global__ void __launch_bounds__(kBlock, 8) rhs_kernel(RhsArgs a) {
     __shared__ __align__(16) unsigned char smem[Smem<T>::kBytes];
-    const int nh = a.n_heavy - a.n_apart;
     const int b = blockIdx.x;
-    if (b < nh) {
-        block_row<T, VK, EK, MODE>(a, a.n_apart + b, smem);
-    } else {
-        window_block<T, VK, EK, MODE>(a, b - nh, smem);
+    if constexpr (sizeof(T) == 4) {
+        const int nh = a.n_heavy - a.n_apart;
+        if (b < nh) block_row<T, VK, EK>(a, a.n_apart + b, smem);
+        else window_block<T, VK, EK>(a, b - nh, smem);
+    } else {  // FP64 heavy rows are all launched apart
+        window_block<T, VK, EK>(a, b, smem);
     }
 }
 
@@ -298,7 +267,7 @@ __global__ void __launch_bounds__(kBlock, 1) heavy_solo_kernel(RhsArgs a) {
         solo_row_fp64<VK, EK, MODE>(a, blockIdx.x, tile, sh);
     } else {
         extern __shared__ __align__(16) unsigned char smem_dyn[];
-        block_row<T, VK, EK, MODE>(a, blockIdx.x, smem_dyn);
+        block_row<T, VK, EK>(a, blockIdx.x, smem_dyn);
     }
 }
 
@@ -341,20 +310,7 @@ cudaError_t launch_typed(const RhsArgs& a, cudaStream_t s) {
     if (a.heavy_only) return launch_heavy_typed<T, VK, EK>(a, s);
     const int grid = a.n_heavy - a.n_apart + a.n_windows;
     if (grid == 0) return cudaSuccess;
-    if constexpr (sizeof(T) == 4) {
-        rhs_kernel<T, VK, EK, kModeTree><<<grid, kBlock, 0, s>>>(a);
-    } else {
-        switch (a.mode) {
-            case kModeNative:
-                rhs_kernel<T, VK, EK, kModeNative><<<grid, kBlock, 0, s>>>(a);
-                break;
-            case kModeTree:
-                rhs_kernel<T, VK, EK, kModeTree><<<grid, kBlock, 0, s>>>(a);
-                break;
-            default:
-                rhs_kernel<T, VK, EK, kModeExact><<<grid, kBlock, 0, s>>>(a);
-        }
-    }
+    rhs_kernel<T, VK, EK><<<grid, kBlock, 0, s>>>(a);
     return cudaGetLastError();
 }
 
