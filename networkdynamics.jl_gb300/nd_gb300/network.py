@@ -451,18 +451,18 @@ def jacobian(nw: Network, u, p, t=0.0, stream=None):
         nw._jac_index = (tuple(torch.from_numpy(x.astype(np.int64)).to(u.device) for x in (rowptr, colidx)),
                          _raw_stream(None))
     index, home = nw._jac_index
+    raw = _raw_stream(stream)
     if stream is not None and not isinstance(stream, torch.cuda.Stream):
-        stream = torch.cuda.ExternalStream(stream.cuda_stream, device=u.device)
+        stream = torch.cuda.ExternalStream(raw, device=u.device)
     # every tensor of the result belongs to the stream that fills it
     with contextlib.nullcontext() if stream is None else torch.cuda.stream(stream):
-        if _raw_stream(None) != home:  # the copies below may outlive the network
+        if raw != home:  # the copies below may outlive the network
             for x in index:
                 x.record_stream(torch.cuda.current_stream())
         crow, col = (x.clone() for x in index)
         values = torch.empty(col.numel(), dtype=u.dtype, device=u.device)
     pp = p.data_ptr() if p is not None and p.numel() else None
-    capi.check(nw._lib.nd_jacobian(nw.handle, _dtype_code(u.dtype), values.data_ptr(), u.data_ptr(), pp, float(t),
-                                   _raw_stream(stream)))
+    capi.check(nw._lib.nd_jacobian(nw.handle, _dtype_code(u.dtype), values.data_ptr(), u.data_ptr(), pp, float(t), raw))
     return torch.sparse_csr_tensor(crow, col, values, size=(nw.dim, nw.dim))
 
 
