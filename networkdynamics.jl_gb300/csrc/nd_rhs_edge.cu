@@ -466,11 +466,13 @@ cudaError_t launch_typed(const RhsArgs& a, cudaStream_t s, int phases) {
     const auto blocks = [](int64_t n, int per) { return (unsigned)((n + per - 1) / per); };
     // Rows start beside the edge phase's last blocks only where y stays in L2: on BA(1e7, 4), with
     // the grouped copy, they took the whole RHS from 743 to 768 µs in FP64 and from 474 to 490 in
-    // FP32 (up to 96 MiB of y they save 3-6 µs of 50-130).  Nor the long FP64 rows of dense networks:
-    // their few one-warp blocks would go several to the first SMs that fall free, whose one FP64
-    // unit their chains of adds then share (WS(3000, 1500) rewired by 0.3, with line weights 152 µs,
-    // with sines 162; after the edge phase 133 and 142.  WS(1900, 950) 84 and 86).
-    const bool early = a.direct && !(a.dense_rows && sizeof(T) == 8);
+    // FP32 (up to 96 MiB of y they save 3-6 µs of 50-130).  Nor, behind an edge phase of some length,
+    // the long FP64 rows of dense networks: their few one-warp blocks would go several to the first SMs
+    // that fall free, whose one FP64 unit their chains of adds then share.  WS(n, n / 2) rewired by
+    // 0.3, early / after the edges' end, µs, with line weights and with sines: n = 1500 65.9 / 67.9 and
+    // 69.9 / 74.0, 1900 84.3 / 86.3 and 100 / 90, 2000 102 / 90 and 106 / 94, 3000 152 / 133 and
+    // 162 / 142.
+    const bool early = a.direct && !(a.dense_rows && sizeof(T) == 8 && a.ne >= 750000);
     const auto launch = [&](void (*k)(RhsArgs), unsigned grid, int block) {
         if (early) return launch_secondary(k, grid, block, s, a);
         k<<<grid, block, 0, s>>>(a);
