@@ -406,14 +406,15 @@ __global__ void __launch_bounds__(kRowBlock) batched_edge_kernel2(BatchedKArgs a
 // Everything that does not need y2 -- the term indices, the vertex's state and parameters, the
 // generators' divisions and sines -- comes before the wait for the edge kernel, whose last
 // blocks are still running then.  Powergrid WS(1e5, 2): edges and rows 27.7 µs before, 24.3 so,
-// of which the FP64 pipe is busy 12.7.  A hub's row is a chain of round trips, one per batch:
-// BA(50000, 2), FP64 / FP32, 115 / 52 µs with batches of four asked for when their turn came,
-// 94 / 42 asked for one batch ahead, 77 / 31 with six (eight: 74 / 27, but small grids 1 µs slower).
+// of which the FP64 pipe is busy 12.7.  The first four terms, most rows' only ones, come by
+// themselves; a longer row is a chain of round trips, one per batch, so its batch of six is on its
+// way while the one before is added: BA(50000, 2), FP64 / FP32, 111 / 50 µs with batches of four
+// asked for when their turn came, 64 / 29 so; WS(300, 2) 6.7 µs either way, 7.1 with six first terms.
 template <typename T>
 __global__ void __launch_bounds__(kRowBlock) batched_row_kernel2(BatchedKArgs a) {
     using A = Arith<T>;
     using V2 = typename Vec2<T>::type;
-    constexpr int kB = 6;
+    constexpr int kB = 4, kD = 6;
     const V2* __restrict__ y2 = static_cast<const V2*>(a.y2);
     const int64_t slot = (int64_t)blockIdx.x * kRowBlock + threadIdx.x;
     if (slot >= a.nv) return;
@@ -440,20 +441,14 @@ __global__ void __launch_bounds__(kRowBlock) batched_row_kernel2(BatchedKArgs a)
     const uint64_t pol = policy_evict_normal();
     wait_for_primary();
     T re = T(0), im = T(0);
-    V2 t[kB], nxt[kB];  // a batch's terms are on their way while the one before is added
+    {
+        V2 t[kB];
 #pragma unroll
-    for (int k = 0; k < kB; ++k) t[k] = ld_edge(y2 + idx[k], pol, k < n);
-#pragma unroll
-    for (int k = 0; k < kB; ++k) idx[k] = kB + k < n ? __ldg(a.tidx + t0 + kB + k) : 0;
-    for (int j0 = 0; j0 < n; j0 += kB) {
-#pragma unroll
-        for (int k = 0; k < kB; ++k) nxt[k] = ld_edge(y2 + idx[k], pol, j0 + kB + k < n);
-#pragma unroll
-        for (int k = 0; k < kB; ++k) idx[k] = j0 + 2 * kB + k < n ? __ldg(a.tidx + t0 + j0 + 2 * kB + k) : 0;
+        for (int k = 0; k < kB; ++k) t[k] = ld_edge(y2 + idx[k], pol, k < n);
 #pragma unroll
         for (int k = 0; k < kB; ++k) {
-            if (j0 + k >= n) break;
-            if (j0 + k == 0) {  // the reference's zero start folded into the first term
+            if (k >= n) break;
+            if (k == 0) {  // the reference's zero start folded into the first term
                 re = zero_plus(t[0].x);
                 im = zero_plus(t[0].y);
             } else {
@@ -461,8 +456,30 @@ __global__ void __launch_bounds__(kRowBlock) batched_row_kernel2(BatchedKArgs a)
                 im = A::add(im, t[k].y);
             }
         }
+    }
+    if (n > kB) {
+        int32_t id[kD];
+        V2 t[kD], nxt[kD];
 #pragma unroll
-        for (int k = 0; k < kB; ++k) t[k] = nxt[k];
+        for (int k = 0; k < kD; ++k) id[k] = kB + k < n ? __ldg(a.tidx + t0 + kB + k) : 0;
+#pragma unroll
+        for (int k = 0; k < kD; ++k) t[k] = ld_edge(y2 + id[k], pol, kB + k < n);
+#pragma unroll
+        for (int k = 0; k < kD; ++k) id[k] = kB + kD + k < n ? __ldg(a.tidx + t0 + kB + kD + k) : 0;
+        for (int j0 = kB; j0 < n; j0 += kD) {
+#pragma unroll
+            for (int k = 0; k < kD; ++k) nxt[k] = ld_edge(y2 + id[k], pol, j0 + kD + k < n);
+#pragma unroll
+            for (int k = 0; k < kD; ++k) id[k] = j0 + 2 * kD + k < n ? __ldg(a.tidx + t0 + j0 + 2 * kD + k) : 0;
+#pragma unroll
+            for (int k = 0; k < kD; ++k) {
+                if (j0 + k >= n) break;
+                re = A::add(re, t[k].x);
+                im = A::add(im, t[k].y);
+            }
+#pragma unroll
+            for (int k = 0; k < kD; ++k) t[k] = nxt[k];
+        }
     }
     if (bus) {
         const Cx<T> uc = cdiv<T>(power, {re, -im});
