@@ -376,17 +376,21 @@ __global__ void __launch_bounds__(NT) batched_row_kernel(BatchedKArgs a, int64_t
 // The same two launches with complex values: y2 holds (y_src, y_dst) as two complex numbers
 // per edge position, a term index t names the complex number y2[t], and a row's real and
 // imaginary parts are summed side by side in the sequential order, one thread per row.
-// Bound by the FP64 pipe (27 operations a line) behind three dependent loads.  Blocks of
+// Bound by the FP64 pipe (27 operations a line) behind three dependent loads.  FP64 in blocks of
 // kRowBlock threads: 1e5 lines are 2.6 blocks of 256 per SM, so some SMs had half as much again
-// to do as others.
+// to do as others.  FP32, bound by its loads, in blocks of 256: grids of 1.5e5, 3e5 and 6e5 buses
+// with lines to 4 others 8.0, 13.6 and 26.1 µs a call, 11.1, 19.5 and 37.1 with blocks of 64.
 template <typename T>
-__global__ void __launch_bounds__(kRowBlock) batched_edge_kernel2(BatchedKArgs a) {
+constexpr int kLineBlock = sizeof(T) == 4 ? kBlock : kRowBlock;
+template <typename T>
+__global__ void __launch_bounds__(kLineBlock<T>) batched_edge_kernel2(BatchedKArgs a) {
     using V2 = typename Vec2<T>::type;
     dependents_may_start();
     const T* __restrict__ u = static_cast<const T*>(a.u);
     const T* __restrict__ p = static_cast<const T*>(a.p);
     V2* __restrict__ y2 = static_cast<V2*>(a.y2);
-    for (int64_t k = (int64_t)blockIdx.x * kRowBlock + threadIdx.x; k < a.ne; k += (int64_t)gridDim.x * kRowBlock) {
+    for (int64_t k = (int64_t)blockIdx.x * kLineBlock<T> + threadIdx.x; k < a.ne;
+         k += (int64_t)gridDim.x * kLineBlock<T>) {
         const int2 uv = __ldg(a.eu + k);
         const int b = find_batch(a.eb, k);  // every edge batch is a pi-line batch
         const int64_t q = __ldg(a.eb.p0 + b) + 4 * (k - __ldg(a.eb.pos0 + b));
@@ -521,8 +525,8 @@ cudaError_t launch_typed(const BatchedNet& b, void* du, const void* u, const voi
     };
     if (b.depth == 2) {
         if ((phases & kPhaseEdge) && b.ne > 0) {
-            const int64_t blocks = std::min<int64_t>((b.ne + kRowBlock - 1) / kRowBlock, int64_t(1) << 20);
-            batched_edge_kernel2<T><<<(unsigned)blocks, kRowBlock, 0, s>>>(a);
+            const int64_t blocks = std::min<int64_t>((b.ne + kLineBlock<T> - 1) / kLineBlock<T>, int64_t(1) << 20);
+            batched_edge_kernel2<T><<<(unsigned)blocks, kLineBlock<T>, 0, s>>>(a);
         }
         if (phases & kPhaseRow)
             return launch_rows(batched_row_kernel2<T>, (b.nv + kRowBlock - 1) / kRowBlock, kRowBlock, a);
