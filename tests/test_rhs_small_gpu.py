@@ -100,3 +100,34 @@ def test_f32_hubs_of_small_networks(cuda, degrees, vk, ek):
     got, ref = gpu_rhs(nw, u, p, cuda, np.float32), on.rhs(u.astype(np.float64), p.astype(np.float64))
     assert np.all(np.abs(got - ref) <= 4e-6 * (on.abs_terms(u.astype(np.float64), p.astype(np.float64)) + np.abs(ref)))
     assert nw.kernel_times()["heavy_rows"][0] == int(max(degrees) > 8192)
+
+
+@pytest.mark.parametrize("long_rows", [1, 3, 4, 5, 6, 31, 40])  # marked by their warp up to four, by a thread above
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_windows_of_long_rows(cuda, long_rows, dtype):
+    """Windows with few and with many rows above 32 terms: the oracle's bits in FP64, FP32 within 4e-6
+    of the term scale."""
+    import torch
+    g = hubs([33 + 7 * i % 60 for i in range(long_rows)], 1500)
+    on = O.OracleNetwork.from_graph(g, O.V_DIFFUSION, O.E_DIFFUSION)
+    u, p = random_inputs(on, O.V_DIFFUSION, np.random.default_rng(long_rows), dtype)
+    nw = nd.adapt(nd.Network(g, nd.diffusion_vertex(), nd.diffusion_edge()),
+                  torch.float64 if dtype == np.float64 else torch.float32)
+    got, ref = gpu_rhs(nw, u, p, cuda, dtype), on.rhs(u.astype(np.float64), p.astype(np.float64))
+    if dtype == np.float64:
+        np.testing.assert_array_equal(got, ref)
+    else:
+        assert np.all(np.abs(got - ref) <= 4e-6 * on.abs_terms(u.astype(np.float64), p.astype(np.float64)))
+
+
+@pytest.mark.parametrize("order", ["sequential", "sequential_hw"])
+@pytest.mark.parametrize("first", [257, 509, 1023])  # remainders of 16 terms; the ends of a tile
+def test_heavy_row_remainders(cuda, first, order):
+    """Heavy rows of every remainder, by the scan and by hardware adds: the oracle's bits."""
+    import torch
+    g = hubs([first + i for i in range(18)], 1500)
+    on = O.OracleNetwork.from_graph(g, O.V_DIFFUSION, O.E_DIFFUSION)
+    u, p = random_inputs(on, O.V_DIFFUSION, np.random.default_rng(first))
+    nw = nd.adapt(nd.Network(g, nd.diffusion_vertex(), nd.diffusion_edge()), torch.float64)
+    nw.set_sum_order(order)
+    np.testing.assert_array_equal(gpu_rhs(nw, u, p, cuda, np.float64), on.rhs(u, p))

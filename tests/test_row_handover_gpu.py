@@ -135,3 +135,30 @@ def test_network_without_edges(cuda, vertices, nv):
     np.testing.assert_array_equal(got.cpu().numpy(), ref)
     uT, _ = solve_tsit5(nw, torch.from_numpy(0.1 * us[0]).to(cuda), pt, (0.0, 0.5), reltol=1e-8, abstol=1e-10)
     assert torch.isfinite(uT).all()
+
+
+@pytest.mark.parametrize("degrees", [tuple(range(18, 36)), (3, 4, 5, 9, 10, 11, 15, 16, 17, 64, 700)])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_powergrid_hubs(cuda, degrees, dtype):
+    """Rows of more lines than the first batch and the next ones hold: the oracle's bits in FP64; FP32
+    as near to it as its own rounding of sums of `n` currents and one division allows."""
+    import torch
+    g = hub_graph(list(degrees), 900)
+    net = nd.Network(g, [nd.pqnode()] * g.nv, nd.piline())
+    on = O.OracleNetwork.from_batches(g.nv, g.src, g.dst, [m.kind for m in net.vertex_batches], net.vertex_batch,
+                                      [(O.E_PILINE, O.C_FIDUCIAL)], net.edge_batch)
+    rng = np.random.default_rng(len(degrees))
+    u, p = rng.normal(size=net.dim).astype(dtype), rng.uniform(0.5, 1.5, size=net.pdim).astype(dtype)
+    got = gpu_rhs(nd.adapt(net, torch.float64 if dtype == np.float64 else torch.float32), u, p, cuda, dtype)
+    ref = on.rhs(u.astype(np.float64), p.astype(np.float64))
+    rows = np.flatnonzero(g.degree())
+    at = np.stack([2 * rows, 2 * rows + 1])
+    if dtype == np.float64:
+        np.testing.assert_array_equal(got[at], ref[at])
+        return
+    # du = S / conj(i): the relative error of |i|, whose n currents (|V| <= 5, 1 / |Z| <= 1.5) sum to
+    # |i| with an error of n (n + 8) 2^-24 * 10, and 16 roundings of the division
+    n, s = g.degree()[rows], np.hypot(*p[:2 * g.nv].astype(np.float64).reshape(-1, 2)[rows].T)
+    size = np.hypot(*ref[at])
+    current = s / size
+    assert np.all(np.hypot(*(got[at].astype(np.float64) - ref[at])) <= size * (n * (n + 8.0) * 10 / current + 16) * 2.0 ** -24)
