@@ -92,11 +92,15 @@ enum nd_edge_kind {
  * Static kinds take the first three; ND_FIDUCIAL is the only coupling of the ODE kinds. */
 enum nd_coupling { ND_ANTISYMMETRIC = 1, ND_SYMMETRIC = 2, ND_DIRECTED = 3, ND_FIDUCIAL = 4 };
 
-/* Summation order of the per-vertex edge aggregation. */
+/* Summation order of the per-vertex edge aggregation, an option of the FP64 heavy rows: those
+ * above 2048 terms, or from 129 to 2049 terms on by the network's size, or from 257 terms on
+ * networks of one launch (see nd_set_layout); where that would be more than an eighth of all
+ * incidences, those above 2048 terms.  Batched networks: rows above 2048 terms.  Shorter rows are
+ * summed in sequence with hardware adds in every order. */
 enum nd_sum_order {
     ND_ORDER_SEQUENTIAL = 0,   /* ascending out-buffer index, = SequentialAggregator (bitwise);
-                                  FP64 adds run as exact integer arithmetic, hubs as an exact scan */
-    ND_ORDER_TREE = 1,         /* deterministic tree inside a warp at hubs (not bitwise)          */
+                                  heavy rows by an exact integer scan                             */
+    ND_ORDER_TREE = 1,         /* heavy rows by a deterministic tree (not bitwise)                */
     ND_ORDER_SEQUENTIAL_HW = 2 /* the sequential order with hardware FP64 adds (bitwise, slower on
                                   GB300, whose FP64 pipe is 1/64 of FP32)                         */
 };
@@ -226,8 +230,8 @@ int nd_set_layout(nd_handle* h, int layout);
 enum nd_kernel_kind {
     ND_KERNEL_EDGE_PHASE = 0, /* one thread per edge: edge outputs y, bucketed by destination */
     ND_KERNEL_ROW_PHASE = 1,  /* row sums over y + vertex functions (all but the heavy rows) */
-    ND_KERNEL_HEAVY_ROWS = 2, /* rows of degree > 2048 (FP64: > 128 to 2048 by size), a block per row
-                                 on the side stream */
+    ND_KERNEL_HEAVY_ROWS = 2, /* heavy rows (see nd_sum_order; FP32: above 2048 terms, on networks of
+                                 one launch above 8192), a block per row on the side stream */
     ND_KERNEL_FUSED = 3,      /* single-kernel RHS (ND_LAYOUT_FUSED or non-canonical edges) */
     ND_KERNEL_BATCHED_EDGES = 4, /* batched networks: edge functions of every edge batch */
     ND_KERNEL_BATCHED_ROWS = 5,  /* batched networks: row sums + vertex functions */

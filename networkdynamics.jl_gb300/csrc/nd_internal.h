@@ -66,14 +66,15 @@ inline int edge_pdim(int ek) {
 inline int vertex_outdim(int vk) { return vk == ND_V_PQ || vk == ND_V_GENERATOR || vk == ND_V_PQ_CONST ? 2 : 1; }
 inline int edge_outdim(int ek) { return ek == ND_E_PILINE ? 2 : 1; }
 
-// Degree buckets.  Rows with degree <= kMediumMaxDeg are processed in windows: a block
-// evaluates all edge terms of up to kWindow rows / kWindowIncidences incidences in
-// parallel, then sums one row per thread; rows are sorted by degree inside a window so
-// the lanes of a warp walk rows of nearly equal length.  Medium rows (degree above
+// Degree buckets.  Rows below the heavy ones (at most kMediumMaxDeg terms) are processed in
+// windows: a block evaluates all edge terms of up to kWindow rows / kWindowIncidences
+// incidences in parallel, then sums one row per thread; rows are sorted by degree inside a
+// window so the lanes of a warp walk rows of nearly equal length.  Medium rows (degree above
 // kLightMaxDeg) come first, globally sorted by degree; light rows follow in runs of
 // kLightRun consecutive vertices, sorted by degree inside each run.
-// Longer rows (power-law hubs) get a block each and are summed by an exact parallel scan:
-// a per-thread chain that long would wait on the shared FP64 pipe at every step.
+// Heavy rows (power-law hubs; heavy_min_deg, kFusedMaxRow) get a block each and are summed by
+// an exact parallel scan: a per-thread chain that long would wait on the shared FP64 pipe at
+// every step.
 constexpr int kLightMaxDeg = 32;
 constexpr int kMediumMaxDeg = 2048;
 // Shortest heavy row of an FP64 handle's two-phase layout with ninc incidences.  A thread sums
@@ -91,7 +92,7 @@ constexpr int64_t heavy_min_deg(int64_t ninc) {
 // trip of its value through memory.  Fused / two-phase, µs per RHS call:
 //   FP64  Kuramoto WS(1e3, 10) 5.8 / 16.5, WS(2e5, 10) 28.8 / 28.8, swing BA(1e4, 2) 20.6 / 24.4,
 //         diffusion BA(2e5, 4) 44.5 / 46.1, BA(5e5, 4) 58.3 / 53.5
-//   FP32  Kuramoto WS(1e3, 10) 5.9 / 12.4, swing BA(1e5, 2) 14.4 / 20.6, diffusion BA(5e5, 4) 34.4 / 35.7
+//   FP32  Kuramoto WS(1e3, 10) 5.9 / 12.4, swing BA(1e5, 2) 10.4 / 20.6, diffusion BA(5e5, 4) 34.4 / 35.7
 // Not in FP64 where rows above kFusedDenseRow terms hold most incidences (a dense graph, whose
 // rows have a prefetching kernel in the two-phase layout): WS(1000, 500) 28.7 / 34.9, WS(1900, 950)
 // 75.9 / 55.4.
@@ -227,13 +228,13 @@ struct RhsArgs {
 
 // Launch the fused RHS for the given element type.
 cudaError_t launch_rhs(int dtype, const RhsArgs& a, cudaStream_t stream);
-// Launch the two-phase (edge-centric) RHS: phase E, phase R or both (kPhase* bits).
 // FP32 rows of ODE-edge networks with at least this many edges run on the handle's side stream
 // beside the edge kernel (WS(3000, 1500): 28.8 µs one after the other, 23.5 beside; WS(1500, 750)
 // 14.4 and 11.2).  Below, the four event calls cost more than the shorter kernel.  Not in FP64,
 // where the rows' chains of adds then wait for the edges' operations in the SM's one FP64 unit
 // (109 µs one after the other, 172 beside).
 constexpr int64_t kOverlapRowsMinEdges = 200000;
+// Launch the two-phase (edge-centric) RHS: phase E, phase R or both (kPhase* bits).
 enum : int { kPhaseEdge = 1, kPhaseRow = 2, kPhaseBoth = 3 };
 cudaError_t launch_rhs_edge(int dtype, const RhsArgs& a, cudaStream_t stream, int phases = kPhaseBoth);
 

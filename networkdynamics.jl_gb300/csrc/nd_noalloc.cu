@@ -140,8 +140,9 @@ __global__ void static_row_kernel(int64_t nv, int64_t ne, const int32_t* __restr
                 s1 = s0;
             }
         }
-        // FP32 rows longer than kLightMaxDeg add with Kahan compensation, as the row phase of
-        // nd_rhs does: both give the same bits on every row of degree <= kMediumMaxDeg
+        // FP32 rows longer than kLightMaxDeg add with Kahan compensation, as nd_rhs does: both give
+        // the same bits on every row of fewer than kWarpRowMinF32 terms, which nd_rhs sums by a
+        // thread (longer ones by a warp or a block)
         const bool kahan = sizeof(T) == 4 && (d1 - d0) + (s1 - s0) > (uint32_t)kLightMaxDeg;
         T acc = T(0), comp = T(0);
         auto add = [&](T term) {

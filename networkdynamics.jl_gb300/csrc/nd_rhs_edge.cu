@@ -10,8 +10,7 @@
 //   R  one thread per row: the row's destination-side values (edges (s, v), s < v, in
 //      ascending edge id) followed by the negated values of its own source block, which
 //      is exactly the order of the vertex's entries in the reference's output buffer, then
-//      vertex f.  Rows of degree above kMediumMaxDeg run in the heavy-row kernel of the
-//      fused path (nd_rhs.cu) on a side stream.
+//      vertex f.  Heavy rows run in a kernel of their own (nd_rhs.cu) on a side stream.
 // The edge function and its FP64 operations run once per edge instead of once per
 // incidence, edge parameters and incidence data are read in order, and the random
 // traffic shrinks to the gather of u[dst] (kept in L2) and the bucket-local gathers of

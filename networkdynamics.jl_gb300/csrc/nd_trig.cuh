@@ -18,7 +18,9 @@
 // used only where that is below 2^-61 of it, so the result is within 0.51 ulp of the exact
 // one (the tests hold 0.51; the library's sine has up to 1 ulp).  Arguments of 2^17 and
 // beyond, infinities, NaN and reduced arguments too close to zero for their error (one in
-// about 10^5) go to the library function.  Both functions are exactly odd / even.
+// about 10^5) go to the library function; so do the products with a factor of 0, below 2^-959, of
+// 2^960 and beyond, or not finite (a line of weight 0 costs a library sine), whose exponents the
+// product in one rounding does not cover.  Both functions are exactly odd / even.
 //
 // The header compiles as CUDA (device) and as plain C++ (host, for the CPU self-test), with
 // the same bits on both for every argument that does not go to the library function.

@@ -76,8 +76,8 @@ parameters, because a Network rebuilds its style from its type (`executionstyle(
 src/network_structure.jl:83-116):
 
 - `sum_order`: `:sequential` (SequentialAggregator's bits), `:sequential_hw` (the same bits,
-  hardware adds at hubs) or `:tree` (deterministic warp tree at hubs, not bitwise);
-- `layout`: `:auto` (two-phase kernels for canonical edge lists) or `:fused`.
+  hardware adds at heavy rows) or `:tree` (a deterministic tree at heavy rows, not bitwise);
+- `layout`: `:auto` (two-phase kernels for canonical edge lists of large networks) or `:fused`.
 
 They are applied to the device handle at adapt time.
 """

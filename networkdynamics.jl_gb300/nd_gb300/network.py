@@ -36,15 +36,17 @@ class GB300Execution(ExecutionStyle):
     src/executionstyles.jl:13-52):
 
     - ``sum_order``: "sequential" (default; the bits of SequentialAggregator, with the exact
-      scan at hubs), "sequential_hw" (the same bits with hardware adds at hubs) or "tree"
-      (a deterministic warp tree at hubs; not bitwise);
+      scan at heavy rows), "sequential_hw" (the same bits with hardware adds there) or "tree"
+      (a deterministic tree there; not bitwise);
     - ``layout``: "auto" (two-phase edge-centric kernels for canonical edge lists of large
       networks, else the fused kernel) or "fused";
     - ``kernel_timing``: bracket every kernel with CUDA events for ``Network.kernel_times``.
 
-    The precision is the dtype given to ``adapt``.  The degree buckets (light rows up to 32,
-    heavy rows above 2048, in FP64 already above 128 to 2048 terms by the network's size) and
-    the FP32 Kahan threshold (rows longer than 32) are constants of the library."""
+    The precision is the dtype given to ``adapt``.  Heavy rows are those above 2048 terms; in
+    FP64 those from 129 to 2049 terms on, by the network's size; on networks that take one
+    launch those from 257 (FP64) or 129 (FP32) terms on.  Where such rows hold more than an eighth
+    of an FP64 network's incidences, only those above 2048 terms are.  These limits and the FP32
+    Kahan threshold (rows longer than 32) are the library's, not options."""
 
     buffered = False
     SUM_ORDERS = ("sequential", "sequential_hw", "tree")
